@@ -15,6 +15,7 @@
 #include "../../include/glmasr_fp4.h"
 #include "elementwise.cuh"
 #include "gemm_simt.cuh"
+#include "gemm_skinny.cuh"
 #include "gemm_umma.cuh"
 #include "runtime.cuh"
 
@@ -550,6 +551,68 @@ static const __nv_bfloat16 *resident_bf16_weight(const glmasr_fp4_weight &w, int
     return r.w;
 }
 
+// Rows that choose between routes with different summation orders.
+static int route_rows(const FusedArgs &a) { return a.M > g_route_rows ? a.M : g_route_rows; }
+
+static bool skinny_eligible(const FusedArgs &a) {
+    if (a.mode == GEMM_BF16 || a.pre != nullptr || a.xq != nullptr || a.q_out != nullptr) return false;
+    if (a.mode == GEMM_W4A4 && (route_rows(a) > 8 || a.num_w != 1 || a.epi != EPI_STORE)) return false;
+    int rows[kMaxSegments];
+    for (int i = 0; i < a.num_w; ++i) rows[i] = a.w[i].N;
+    return skinny_covers(route_rows(a), a.K, rows, a.num_w, a.epi);
+}
+
+static int run_skinny(const FusedArgs &a, const __nv_bfloat16 *norm_w = nullptr, float eps = 0.0f) {
+    SkinnyParams p;
+    memset(&p, 0, sizeof(p));
+    p.x = a.x;
+    p.ldx = a.ldx;
+    p.M = a.M;
+    p.K = a.K;
+    p.norm_w = norm_w;
+    p.eps = eps;
+    p.inv_in = a.mode == GEMM_W4A4 ? 1.0f / a.input_scale : 0.0f;
+    double n_rows = 0.0;
+    for (int i = 0; i < a.num_w; ++i) {
+        p.w[i] = a.w[i].w_packed;
+        p.ws[i] = a.w[i].w_scales;
+        p.seg_rows[i] = a.w[i].N;
+        p.alpha[i] = a.mode == GEMM_W4A4 ? a.input_scale * a.w[i].w_global_scale : a.w[i].w_global_scale;
+        n_rows += a.w[i].N;
+    }
+    p.num_segs = a.num_w;
+    p.epi = a.epi;
+    p.out = a.out;
+    p.residual = a.residual;
+    p.bias = a.bias;
+    p.ldo = a.ldo;
+    p.status = device_status_word();
+    profile_bracket_begin(2.0 * a.M * n_rows * a.K, 0.5625 * n_rows * a.K + 2.0 * a.M * (a.K + total_out_cols(a)));
+    if (launch_skinny_linear(p, num_sms(), g_stream) != cudaSuccess) return -1;
+    profile_bracket_end();
+    ++g_launches;
+    return 0;
+}
+
+// RMSNorm (eps) of x [M, K] with norm_w, then up to three W4A16 projections of it, as one launch.  -1: not covered.
+int fp4_linear_w4a16_normed(uint16_t *out, int ldo, const uint16_t *x, const uint16_t *norm_w, float eps,
+                            const glmasr_fp4_weight *weights, int num_weights, int epilogue, int M, int K) {
+    FusedArgs a;
+    memset(&a, 0, sizeof(a));
+    a.mode = GEMM_W4A16;
+    a.out = (__nv_bfloat16 *)out;
+    a.ldo = ldo;
+    a.x = (const __nv_bfloat16 *)x;
+    a.ldx = K;
+    a.w = weights;
+    a.num_w = num_weights;
+    a.epi = epilogue;
+    a.M = M;
+    a.K = K;
+    if (!tensor_core_eligible(a) || !aligned16(norm_w) || !skinny_eligible(a)) return -1;
+    return run_skinny(a, (const __nv_bfloat16 *)norm_w, eps);
+}
+
 static int run_fused(const FusedArgs &a) {
     if (a.M <= 0 || a.K <= 0) return -1;
     if (a.mode != GEMM_BF16) {
@@ -564,6 +627,11 @@ static int run_fused(const FusedArgs &a) {
         if (a.xq != nullptr || a.q_out != nullptr) return -1;   // quantised hand-over exists on the tensor-core path only
         return run_simt(a);
     }
+
+    // A handful of rows: the few-row kernel reads the packed weights as they are.  W4A16 takes it up to its 32 rows.  A
+    // single W4A4 linear does up to 8 (every CTA quantises the rows for itself); fused W4A4 projections and quantised
+    // hand-overs, the parts of a chain, stay on the block-scaled MMA whose bits they share with the resident kernel.
+    if (skinny_eligible(a)) return run_skinny(a);
 
     // W4A16 on resident bf16 copies of the weights (made on first use, within the budget): the bf16 GEMM streams
     // them at the rate of the memory system, where the in-kernel dequant of a decode-sized call is a chain of
@@ -590,7 +658,7 @@ static int run_fused(const FusedArgs &a) {
     // W4A16 with many rows: the in-kernel dequant (repeated for every 128-row tile) becomes the
     // bottleneck, so do what the reference does -- dequantise each weight once to bf16
     // (Infer-engine/cuda/kernels.cu:1316) -- and run the bf16 GEMM on the result.
-    if (a.mode == GEMM_W4A16 && (a.M > g_route_rows ? a.M : g_route_rows) >= w4a16_dequant_once_rows()) {
+    if (a.mode == GEMM_W4A16 && route_rows(a) >= w4a16_dequant_once_rows()) {
         size_t elems = 0;
         for (int i = 0; i < a.num_w; ++i) elems += (size_t)a.w[i].N * a.K;
         __nv_bfloat16 *wd = (a.weight_scratch != nullptr && a.num_w == 1)

@@ -21,13 +21,15 @@ namespace glmasr {
 // and all threads normalise.
 // --------------------------------------------------------------------------------------------
 __global__ void rmsnorm_kernel(__nv_bfloat16 *__restrict__ out, const __nv_bfloat16 *__restrict__ x,
-                               const __nv_bfloat16 *__restrict__ weight, float eps, int rows, int dim) {
+                               const __nv_bfloat16 *__restrict__ weight, float eps, int rows, int dim, int *lens_out,
+                               const int *lens_in) {
     pdl_launch_dependents();
     pdl_wait();
     extern __shared__ __nv_bfloat16 row_s[];
     __shared__ float rms_s;
     const int row = blockIdx.x;
     if (row >= rows) return;
+    if (lens_out != nullptr && threadIdx.x == 0) lens_out[row] = lens_in[row];
     const __nv_bfloat16 *xr = x + (size_t)row * dim;
     __nv_bfloat16 *orow = out + (size_t)row * dim;
     const bool vec = (dim % 8 == 0) && (((uintptr_t)xr & 15) == 0) && (((uintptr_t)orow & 15) == 0) &&
@@ -75,7 +77,16 @@ void launch_rmsnorm(__nv_bfloat16 *out, const __nv_bfloat16 *x, const __nv_bfloa
                     int dim, cudaStream_t st) {
     if (rows <= 0 || dim <= 0) return;
     GLMASR_PREFER_MAX_SMEM(rmsnorm_kernel);
-    launch_chained(rmsnorm_kernel, dim3(rows), dim3(256), (size_t)dim * sizeof(__nv_bfloat16), st, out, x, weight, eps, rows, dim);
+    launch_chained(rmsnorm_kernel, dim3(rows), dim3(256), (size_t)dim * sizeof(__nv_bfloat16), st, out, x, weight, eps, rows, dim,
+                   (int *)nullptr, (const int *)nullptr);
+}
+
+void launch_rmsnorm_lens(__nv_bfloat16 *out, const __nv_bfloat16 *x, const __nv_bfloat16 *weight, float eps, int rows, int dim,
+                         int *lens_out, const int *lens_in, cudaStream_t st) {
+    if (rows <= 0 || dim <= 0) return;
+    GLMASR_PREFER_MAX_SMEM(rmsnorm_kernel);
+    launch_chained(rmsnorm_kernel, dim3(rows), dim3(256), (size_t)dim * sizeof(__nv_bfloat16), st, out, x, weight, eps, rows, dim,
+                   lens_out, lens_in);
 }
 
 // --------------------------------------------------------------------------------------------
@@ -670,6 +681,81 @@ __global__ void gather_block_tables_kernel(int *__restrict__ dst, const int *__r
 void launch_gather_block_tables(int *dst, const int *tables, const int *rows, int n, int width, cudaStream_t st) {
     GLMASR_PREFER_MAX_SMEM(gather_block_tables_kernel);
     if (n > 0) launch_chained(gather_block_tables_kernel, dim3(n), dim3(128), 0, st, dst, tables, rows, n, width);
+}
+
+// The host side of a decode step in one launch.  As five copies from pageable memory (each staged by the driver), a row
+// gather, a table gather and the angle kernel it was 20 - 40 us of idle GPU in front of every step; the values fit the
+// parameters of one kernel.
+template <int CAP>
+struct StepSetupParams {
+    const __nv_bfloat16 *rows[CAP];
+    int64_t slot[CAP];
+    int total[CAP], table_row[CAP];
+    __nv_bfloat16 *hidden;
+    int64_t *d_slot;
+    int *d_total, *d_tables;
+    const int *tables, *positions;
+    float *angles;
+    int dim, width, head_dim;
+};
+
+template <int CAP>
+__global__ void __launch_bounds__(256) step_setup_kernel(const __grid_constant__ StepSetupParams<CAP> p) {
+    pdl_launch_dependents();
+    pdl_wait();
+    const int i = blockIdx.x;
+    const uint4 *src = reinterpret_cast<const uint4 *>(p.rows[i]);
+    uint4 *dst = reinterpret_cast<uint4 *>(p.hidden + (size_t)i * p.dim);
+    for (int d = threadIdx.x; d < p.dim / 8; d += blockDim.x) dst[d] = src[d];
+    const int *bt = p.tables + (size_t)p.table_row[i] * p.width;
+    for (int d = threadIdx.x; d < p.width; d += blockDim.x) p.d_tables[(size_t)i * p.width + d] = bt[d];
+    const int half_dim = p.head_dim / 2;
+    for (int d = threadIdx.x; d < half_dim; d += blockDim.x) {       // as rope_angles_kernel
+        const float theta = p.positions[i] * g_inv_freq[d];
+        p.angles[(size_t)i * p.head_dim + d] = cosf(theta);
+        p.angles[(size_t)i * p.head_dim + half_dim + d] = sinf(theta);
+    }
+    if (threadIdx.x == 0) {
+        p.d_slot[i] = p.slot[i];
+        p.d_total[i] = p.total[i];
+    }
+}
+
+template <int CAP>
+static void launch_step_setup_cap(__nv_bfloat16 *hidden, uint16_t *const *rows, int n, int dim, const int64_t *h_slot, int64_t *d_slot,
+                                  const int *h_total, int *d_total, const int *h_table_rows, const int *tables, int *d_tables,
+                                  int width, const int *d_positions, float *angles, int head_dim, cudaStream_t st) {
+    StepSetupParams<CAP> p;
+    for (int i = 0; i < n; ++i) {
+        p.rows[i] = (const __nv_bfloat16 *)rows[i];
+        p.slot[i] = h_slot[i];
+        p.total[i] = h_total[i];
+        p.table_row[i] = h_table_rows[i];
+    }
+    p.hidden = hidden;
+    p.d_slot = d_slot;
+    p.d_total = d_total;
+    p.d_tables = d_tables;
+    p.tables = tables;
+    p.positions = d_positions;
+    p.angles = angles;
+    p.dim = dim;
+    p.width = width;
+    p.head_dim = head_dim;
+    GLMASR_PREFER_MAX_SMEM(step_setup_kernel<CAP>);
+    launch_chained(step_setup_kernel<CAP>, dim3(n), dim3(256), (size_t)0, st, p);
+}
+
+bool launch_step_setup(__nv_bfloat16 *hidden, uint16_t *const *rows, int n, int dim, const int64_t *h_slot, int64_t *d_slot,
+                       const int *h_total, int *d_total, const int *h_table_rows, const int *tables, int *d_tables, int width,
+                       const int *d_positions, float *angles, int head_dim, cudaStream_t st) {
+    if (n < 1 || n > kStepSetupMax || (dim % 8) != 0 || (head_dim % 2) != 0 || head_dim > 1024 || angles == nullptr) return false;
+    for (int i = 0; i < n; ++i)
+        if (((uintptr_t)rows[i] & 15) != 0) return false;
+    ensure_inv_freq(head_dim, st);
+    auto launch = n <= 32 ? launch_step_setup_cap<32> : launch_step_setup_cap<kStepSetupMax>;   // fewer parameters for a small batch
+    launch(hidden, rows, n, dim, h_slot, d_slot, h_total, d_total, h_table_rows, tables, d_tables, width, d_positions, angles, head_dim, st);
+    return true;
 }
 
 }  // namespace glmasr

@@ -46,6 +46,24 @@ bool launch_paged_decode_attention_mma(__nv_bfloat16 *out, int ldo, const __nv_b
                                        int num_kv_heads, int head_dim, int block_size, int max_blocks_per_seq,
                                        cudaStream_t st, uint8_t *q_packed = nullptr, uint8_t *q_sf = nullptr,
                                        float q_input_scale = 0.0f);
+// RoPE + cache write + attention of a small decode batch as one launch, context cut over clusters; angles as
+// launch_rope_angles writes them, max_len = the longest context (tokens attended).  False when another route is better or
+// the layout is not covered (nothing launched).
+bool launch_paged_decode_split(__nv_bfloat16 *out, int ldo, const __nv_bfloat16 *qkv, int ld, int k_col, int v_col,
+                               const float *angles, const int64_t *slot_mapping, __nv_bfloat16 *key_cache,
+                               __nv_bfloat16 *value_cache, const int *block_tables, const int *seq_lens, int num_seqs,
+                               int num_q_heads, int num_kv_heads, int head_dim, int block_size, int max_blocks_per_seq,
+                               int max_len, cudaStream_t st);
+// Everything a decode step needs on the device before its first layer, in one launch: hidden rows gathered from rows[i]
+// (16-byte aligned, dim % 8 == 0), cache slots, lengths, block-table rows and rotary angles of the cached positions.
+// The host values travel as kernel parameters.  False when the batch is too large for that.
+static constexpr int kStepSetupMax = 256;
+bool launch_step_setup(__nv_bfloat16 *hidden, uint16_t *const *rows, int n, int dim, const int64_t *h_slot, int64_t *d_slot,
+                       const int *h_total, int *d_total, const int *h_table_rows, const int *tables, int *d_tables, int width,
+                       const int *d_positions, float *angles, int head_dim, cudaStream_t st);
+// out = rmsnorm(x) as launch_rmsnorm, and lens_out[row] = lens_in[row].
+void launch_rmsnorm_lens(__nv_bfloat16 *out, const __nv_bfloat16 *x, const __nv_bfloat16 *weight, float eps, int rows, int dim,
+                         int *lens_out, const int *lens_in, cudaStream_t st);
 // Variable-length GQA self-attention of a prefill batch (prefill_attention.cu): sequence s owns rows
 // [seq_offsets[s], +seq_lens[s]) of q / k / v / out (device arrays; seq_lens == NULL: seq_offsets is a
 // cumulative table of num_seqs + 1 entries); head_dim 128.  total_tokens = rows of q / k / v (the sequences

@@ -34,6 +34,8 @@ int fp4_linear_w4a4_prequantized(uint16_t *out, int ldo, const uint8_t *xq, cons
                                  const glmasr_fp4_weight *weights, int num_weights, float input_scale, int epilogue,
                                  const uint16_t *residual, int M, int K, uint8_t *q_out = nullptr,
                                  uint8_t *q_out_sf = nullptr, float q_out_input_scale = 0.0f);   // api.cu
+int fp4_linear_w4a16_normed(uint16_t *out, int ldo, const uint16_t *x, const uint16_t *norm_w, float eps,
+                            const glmasr_fp4_weight *weights, int num_weights, int epilogue, int M, int K);   // api.cu
 int fp4_linear_w4a16_silu_quantized(uint8_t *q_out, uint8_t *q_out_sf, float q_out_input_scale, const uint16_t *x, int ldx,
                                     const glmasr_fp4_weight *gate_up, int M, int K);             // api.cu
 
@@ -297,6 +299,18 @@ static void single_proj_prequantized(uint16_t *out, int ldo, const uint8_t *xq, 
     GLMASR_CHECK(rc == 0, "decoder projection on a quantised input failed (N=%d K=%d M=%d)", p.N, p.K, M);
 }
 
+// RMSNorm and same-input W4A16 projections of a few rows as one launch; false when that route does not cover them.
+static bool normed_proj_w4a16(uint16_t *out, int ldo, const uint16_t *x, const uint16_t *norm_w, float eps, const ProjRef *const *ps,
+                              int n, int epi, int M, int H) {
+    if (prefer_w4a4() || !fusable(ps, n) || ps[0]->K != H) return false;
+    glmasr_fp4_weight w[3];
+    for (int i = 0; i < n; ++i) {
+        if (ps[i]->scales == nullptr) return false;
+        w[i] = as_weight(*ps[i]);
+    }
+    return fp4_linear_w4a16_normed(out, ldo, x, norm_w, eps, w, n, epi, M, H) == 0;
+}
+
 // Scratch of one driver call (private workspace slots), shared by the per-layer stages below.
 struct StepBuffers {
     uint16_t *nrm;       // [M, H] bf16: normed hidden state, for consumers that take bf16
@@ -325,7 +339,9 @@ static int project_qkv(const LayerRef &R, const uint16_t *hid, const StepBuffers
         GLMASR_CHECK(ok, "decoder k|v projection failed (M=%d H=%d)", M, H);
         return 1;
     }
-    // (3) everything else: bf16 norm, then whatever can be fused
+    // (3) W4A16 throughout, few rows: norm and projection in one launch
+    if (normed_proj_w4a16(B.qkv, NQKV, hid, R.norm1, 1e-5f, qkv_p, 3, GLMASR_EPI_STORE, M, H)) return 0;
+    // (4) everything else: bf16 norm, then whatever can be fused
     launch_rmsnorm((__nv_bfloat16 *)B.nrm, (const __nv_bfloat16 *)hid, (const __nv_bfloat16 *)R.norm1, 1e-5f, M, H, st);
     // W4A16 throughout: one q|k|v GEMM gives the values of fp4_linear(q) + the fused k|v pair
     if (!prefer_w4a4() && fused_proj(B.qkv, NQKV, B.nrm, H, qkv_p, 3, GLMASR_EPI_STORE, M)) return 1;
@@ -353,8 +369,13 @@ static int project_mlp(const LayerRef &R, uint16_t *hid, const StepBuffers &B, i
         single_proj(hid, H, B.act, F, R.down, M, hid, B.scratch);
         return 0;
     }
+    // (2) W4A16 throughout, few rows: norm, gate|up and SiLU-gate in one launch
+    if (R.gate.N == F && R.up.N == F && normed_proj_w4a16(B.act, F, hid, R.norm2, 1e-5f, gu_p, 2, GLMASR_EPI_SILU_GATE, M, H)) {
+        single_proj(hid, H, B.act, F, R.down, M, hid, B.scratch);
+        return 0;
+    }
     launch_rmsnorm((__nv_bfloat16 *)B.nrm, (const __nv_bfloat16 *)hid, (const __nv_bfloat16 *)R.norm2, 1e-5f, M, H, st);
-    // (2) the reference's mix: gate|up as one W4A16 GEMM (Infer-engine/cuda/decoder.cu:2107-2112) whose SiLU-gate
+    // (3) the reference's mix: gate|up as one W4A16 GEMM (Infer-engine/cuda/decoder.cu:2107-2112) whose SiLU-gate
     //     epilogue writes the native down projection's quantised operand
     if (prefer_w4a4() && !pairs_w4a4() && down_q && fusable(gu_p, 2) && R.gate.K == H && R.gate.N == F && R.up.N == F) {
         const glmasr_fp4_weight gu[2] = {as_weight(R.gate), as_weight(R.up)};
@@ -363,7 +384,7 @@ static int project_mlp(const LayerRef &R, uint16_t *hid, const StepBuffers &B, i
             return 1;
         }
     }
-    // (3) everything else
+    // (4) everything else
     if (!fused_proj(B.act, F, B.nrm, H, gu_p, 2, GLMASR_EPI_SILU_GATE, M)) {
         single_proj(B.act, F, B.nrm, H, R.gate, M, nullptr, B.scratch);
         single_proj(B.act + (size_t)M * F, F, B.nrm, H, R.up, M, nullptr, B.scratch);
@@ -764,6 +785,7 @@ extern "C" void decoder_decode_step_batched(void *handle, const void *ws_v, uint
     std::vector<int64_t> h_slot(M);
     std::vector<int> h_total(M), h_rows(M);
     bool contiguous = true;
+    int max_total = 0;
     for (int s = 0; s < M; ++s) {
         const int cached = h_seq_lens[s];
         GLMASR_CHECK(query_ptrs[s] != nullptr, "decoder_decode_step_batched: query_ptrs[%d] is NULL", s);
@@ -774,6 +796,7 @@ extern "C" void decoder_decode_step_batched(void *handle, const void *ws_v, uint
                      s, cached, bts[s].num_blocks);
         h_slot[s] = (int64_t)bts[s].h_table[logical] * (int64_t)pool->block_size + (int64_t)(cached % pool->block_size);
         h_total[s] = cached + 1;
+        if (cached + 1 > max_total) max_total = cached + 1;
         h_rows[s] = seq_indices ? seq_indices[s] : bts[s].seq_idx;
         GLMASR_CHECK(h_rows[s] >= 0 && h_rows[s] < pool->max_seqs,
                      "decoder_decode_step_batched: invalid seq index %d for batch row %d", h_rows[s], s);
@@ -800,21 +823,27 @@ extern "C" void decoder_decode_step_batched(void *handle, const void *ws_v, uint
 
     const StepBuffers B = {nrm, qkv, act, scratch, nq, nsf, aq, asf};
 
-    GLMASR_CUDA_CHECK(cudaMemcpyAsync(d_slot, h_slot.data(), (size_t)M * sizeof(int64_t), cudaMemcpyHostToDevice, st));
-    GLMASR_CUDA_CHECK(cudaMemcpyAsync(d_total, h_total.data(), (size_t)M * sizeof(int), cudaMemcpyHostToDevice, st));
-    GLMASR_CUDA_CHECK(cudaMemcpyAsync(d_rows, h_rows.data(), (size_t)M * sizeof(int), cudaMemcpyHostToDevice, st));
-    if (contiguous) {
-        GLMASR_CUDA_CHECK(cudaMemcpyAsync(hid, query_ptrs[0], (size_t)M * H * 2, cudaMemcpyDeviceToDevice, st));
-    } else {
-        GLMASR_CUDA_CHECK(cudaMemcpyAsync(d_ptrs, query_ptrs, (size_t)M * sizeof(void *), cudaMemcpyHostToDevice, st));
-        launch_gather_rows((__nv_bfloat16 *)hid, (const __nv_bfloat16 *const *)d_ptrs, M, H, st);
-    }
-    launch_gather_block_tables(d_bt, pool->d_block_tables, d_rows, M, pool->max_blocks_per_seq, st);
-    // the vectors above are pageable host memory: the async copies have completed staging on return
     // the rotary angles depend on the positions only: one evaluation for all layers
     float *rope_angles = (float *)workspace_slot(WS_D_ANGLES, (size_t)M * HD * sizeof(float));
-    if (launch_rope_angles(rope_angles, d_seq_lens, M, HD, st)) note_launches(1);
-    else rope_angles = nullptr;
+    if (launch_step_setup((__nv_bfloat16 *)hid, query_ptrs, M, H, h_slot.data(), d_slot, h_total.data(), d_total, h_rows.data(),
+                          pool->d_block_tables, d_bt, pool->max_blocks_per_seq, d_seq_lens, rope_angles, HD, st)) {
+        note_launches(1);
+        if (!contiguous) GLMASR_CUDA_CHECK(cudaMemcpyAsync(d_ptrs, query_ptrs, (size_t)M * sizeof(void *), cudaMemcpyHostToDevice, st));
+    } else {
+        GLMASR_CUDA_CHECK(cudaMemcpyAsync(d_slot, h_slot.data(), (size_t)M * sizeof(int64_t), cudaMemcpyHostToDevice, st));
+        GLMASR_CUDA_CHECK(cudaMemcpyAsync(d_total, h_total.data(), (size_t)M * sizeof(int), cudaMemcpyHostToDevice, st));
+        GLMASR_CUDA_CHECK(cudaMemcpyAsync(d_rows, h_rows.data(), (size_t)M * sizeof(int), cudaMemcpyHostToDevice, st));
+        if (contiguous) {
+            GLMASR_CUDA_CHECK(cudaMemcpyAsync(hid, query_ptrs[0], (size_t)M * H * 2, cudaMemcpyDeviceToDevice, st));
+        } else {
+            GLMASR_CUDA_CHECK(cudaMemcpyAsync(d_ptrs, query_ptrs, (size_t)M * sizeof(void *), cudaMemcpyHostToDevice, st));
+            launch_gather_rows((__nv_bfloat16 *)hid, (const __nv_bfloat16 *const *)d_ptrs, M, H, st);
+        }
+        launch_gather_block_tables(d_bt, pool->d_block_tables, d_rows, M, pool->max_blocks_per_seq, st);
+        // the vectors above are pageable host memory: the async copies have completed staging on return
+        if (launch_rope_angles(rope_angles, d_seq_lens, M, HD, st)) note_launches(1);
+        else rope_angles = nullptr;
+    }
 
     // the layer tail (o .. next layer's q|k|v) as one co-resident launch where it applies
     const bool tail = tail_enabled() && M <= 256;
@@ -836,6 +865,18 @@ extern "C" void decoder_decode_step_batched(void *handle, const void *ws_v, uint
         // q | k | v into one [M, H + 2 KV] buffer
         int glue = have_qkv ? 0 : project_qkv(R, hid, B, M, H, KV, st);
         have_qkv = false;
+        // attention writes the o projection's quantised operand itself when that projection runs in W4A4
+        const bool o_q = takes_quantised_input(R.o) && R.o.K == H && !attn_scalar_forced();
+        // a small batch whose o projection takes bf16: RoPE, cache write and attention in one launch
+        if (!o_q && !attn_scalar_forced() &&
+            launch_paged_decode_split((__nv_bfloat16 *)att, H, (const __nv_bfloat16 *)qkv, NQKV, H, H + KV, rope_angles, d_slot,
+                                      k_base, v_base, d_bt, d_total, M, QH, KVH, HD, pool->block_size,
+                                      pool->max_blocks_per_seq, max_total, st)) {
+            single_proj(hid, H, att, H, R.o, M, hid, scratch);
+            glue += project_mlp(R, hid, B, M, H, F, st);
+            note_launches(glue + 1);
+            continue;
+        }
         // RoPE on q and k in place (position = cached length), KV write, attention over cached + 1 tokens
         if (launch_rope_qk_cache((__nv_bfloat16 *)qkv, NQKV, H, H + KV, d_seq_lens, d_slot, k_base, v_base, M, QH, KVH, HD, st, rope_angles)) {
             glue += 1;
@@ -846,8 +887,6 @@ extern "C" void decoder_decode_step_batched(void *handle, const void *ws_v, uint
                                      (const __nv_bfloat16 *)qkv + H + KV, NQKV, d_slot, M, KVH, HD, pool->block_size, st);
             glue += 3;
         }
-        // attention writes the o projection's quantised operand itself when that projection runs in W4A4
-        const bool o_q = takes_quantised_input(R.o) && R.o.K == H && !attn_scalar_forced();
         bool ok = false;
         if (o_q)
             ok = launch_paged_decode_attention_mma((__nv_bfloat16 *)att, H, (const __nv_bfloat16 *)qkv, NQKV, k_base, v_base, d_bt,
@@ -873,15 +912,18 @@ extern "C" void decoder_decode_step_batched(void *handle, const void *ws_v, uint
         note_launches(glue + 1);   // norms, RoPE / cache write, attention (the projections count themselves)
     }
 
-    launch_rmsnorm((__nv_bfloat16 *)hid, (const __nv_bfloat16 *)hid, (const __nv_bfloat16 *)refs.final_norm, 1e-5f, M, H, st);
+    // final norm straight into the caller's rows, advanced lengths with it
     if (contiguous) {
-        GLMASR_CUDA_CHECK(cudaMemcpyAsync(query_ptrs[0], hid, (size_t)M * H * 2, cudaMemcpyDeviceToDevice, st));
+        launch_rmsnorm_lens((__nv_bfloat16 *)query_ptrs[0], (const __nv_bfloat16 *)hid, (const __nv_bfloat16 *)refs.final_norm, 1e-5f,
+                            M, H, d_seq_lens, d_total, st);
+        note_launches(1);
     } else {
+        launch_rmsnorm_lens((__nv_bfloat16 *)hid, (const __nv_bfloat16 *)hid, (const __nv_bfloat16 *)refs.final_norm, 1e-5f, M, H,
+                            d_seq_lens, d_total, st);
         launch_scatter_rows((__nv_bfloat16 *const *)d_ptrs, (const __nv_bfloat16 *)hid, M, H, st);
+        note_launches(2);
     }
-    note_launches(2);
     for (int s = 0; s < M; ++s) h_seq_lens[s] = h_total[s];
-    GLMASR_CUDA_CHECK(cudaMemcpyAsync(d_seq_lens, d_total, (size_t)M * sizeof(int), cudaMemcpyDeviceToDevice, st));
     GLMASR_CUDA_CHECK(cudaGetLastError());
 }
 

@@ -1,0 +1,68 @@
+"""The few-row FP4 linear (1 to 32 rows of W4A16, 1 to 8 of a single W4A4 linear) at the edges of its token tiles (8, 16, 32),
+of its 16-row units and of its chunks of K, against the float32 oracles.  Tolerance: one bf16 rounding of the result
+(2^-9) and the order of a float32 sum of at most 8192 exact products, the bar every other route is held to."""
+import numpy as np
+import pytest
+import torch
+
+import fp4_oracle as o
+from gpu_util import REL_TOL_TIGHT, REL_TOL_VS_ORACLE, bits_of, to_dev_bf16, to_dev_u8
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ops():
+    from glm_asr_stack_b200 import ops as _ops
+    yield _ops
+    assert _ops.status() == 0
+
+
+def dev(ops, w):
+    return ops.Fp4Tensor(to_dev_u8(w[0]), to_dev_u8(w[1]), w[2])
+
+
+@pytest.mark.parametrize("M", [1, 7, 8, 9, 16, 17, 32])
+@pytest.mark.parametrize("N,K", [(16, 256), (272, 2048), (48, 8192), (4752, 512)])
+def test_store_and_bias(ops, M, N, K):
+    w, x = o.seeded_weight(N, K, N + K), o.seeded_activation(M, K, M)
+    bias = o.seeded_activation(1, N, 3)[0]
+    d = dev(ops, w)
+    out = bits_of(ops.fp4_linear(to_dev_bf16(x), d.w_packed, d.w_scales, d.w_global_scale, None, to_dev_bf16(bias)))
+    assert o.rel_err(out, o.fp4_linear(x, *w, None, bias)) <= REL_TOL_TIGHT
+    if M <= 8:
+        isc = o.default_input_scale(x)
+        got = torch.empty((M, N), dtype=torch.bfloat16, device="cuda")
+        assert ops.nvfp4_linear(got, to_dev_bf16(x), d.w_packed, d.w_scales, isc, d.w_global_scale) == 0
+        assert o.rel_err(bits_of(got), o.nvfp4_linear(x, w[0], w[1], isc, w[2])) <= REL_TOL_TIGHT
+
+
+@pytest.mark.parametrize("M", [1, 8, 13, 19])
+def test_segments_gate_and_residual(ops, M):
+    K = 512
+    x = o.seeded_activation(M, K, M)
+    ws = [o.seeded_weight(n, K, n) for n in (2384, 32, 80)]
+    out = bits_of(ops.fp4_linear_fused(ops.MODE_W4A16, to_dev_bf16(x), [dev(ops, w) for w in ws]))
+    for w, c in zip(ws, (0, 2384, 2416)):
+        assert o.rel_err(out[:, c:c + w[0].shape[0]], o.linear_o1(x, *w)) <= REL_TOL_TIGHT
+    g, u = o.seeded_weight(2416, K, 5), o.seeded_weight(2416, K, 6)
+    act = bits_of(ops.fp4_linear_fused(ops.MODE_W4A16, to_dev_bf16(x), [dev(ops, g), dev(ops, u)], epilogue=ops.EPI_SILU_GATE))
+    want = o.silu_mul_split_packed(np.concatenate([o.linear_o1(x, *g), o.linear_o1(x, *u)], axis=1))
+    assert o.rel_err(act, want) <= REL_TOL_VS_ORACLE
+    res = to_dev_bf16(o.seeded_activation(M, 2384, 9))
+    want = o.residual_add(o.linear_o1(x, *ws[0]), bits_of(res))
+    ops.fp4_linear_fused(ops.MODE_W4A16, to_dev_bf16(x), [dev(ops, ws[0])], epilogue=ops.EPI_RESIDUAL, residual=res, out=res)
+    assert o.rel_err(bits_of(res), want) <= REL_TOL_TIGHT
+
+
+def test_scale_codes(ops):
+    """Every e4m3 scale byte, subnormal, 0x7F (480 here, not a NaN) and negative ones included, times every e2m1 code."""
+    N, K = 256, 256
+    packed = np.tile(np.arange(128, dtype=np.uint8) * 2 + 1, (N, 1))
+    scales = np.repeat(np.arange(256, dtype=np.uint8)[:, None], K // 16, axis=1)
+    for k0 in (0, 100):
+        x = np.zeros((2, K), np.float32)
+        x[0, k0:k0 + 16], x[1, k0 + 16:k0 + 32:2] = 1.0, -0.5
+        xb = (x.view(np.uint32) >> 16).astype(np.uint16)
+        out = ops.fp4_linear(to_dev_bf16(xb), to_dev_u8(packed), to_dev_u8(scales), 1.0)
+        assert o.rel_err(bits_of(out), o.linear_o1(xb, packed, scales, 1.0)) <= REL_TOL_TIGHT
