@@ -14,6 +14,7 @@
 
 #include "../../include/glmasr_fp4.h"
 #include "elementwise.cuh"
+#include "gemm_cluster.cuh"
 #include "gemm_simt.cuh"
 #include "gemm_skinny.cuh"
 #include "gemm_umma.cuh"
@@ -425,6 +426,8 @@ struct FusedArgs {
     const uint8_t *xq, *xq_sf;
     uint8_t *q_out, *q_out_sf;
     float q_out_input_scale;
+    // BF16 mode: no kernel that may still be running when this call's kernel starts writes the weights
+    bool const_weights;
 };
 
 static bool aligned16(const void *p) { return ((uintptr_t)p & 15) == 0; }
@@ -613,6 +616,60 @@ int fp4_linear_w4a16_normed(uint16_t *out, int ldo, const uint16_t *x, const uin
     return run_skinny(a, (const __nv_bfloat16 *)norm_w, eps);
 }
 
+// GLMASR_CLUSTER_ROWS=n: most rows that the cluster split-K bf16 GEMM takes (comparison runs; 0: never)
+static int cluster_gemm_rows() {
+    static int v = -1;
+    if (v < 0) {
+        const char *e = getenv("GLMASR_CLUSTER_ROWS");
+        v = (e && e[0]) ? atoi(e) : kClusterMaxRows;
+        if (v > kClusterMaxRows) v = kClusterMaxRows;
+        if (v < 0) v = 0;
+    }
+    return v;
+}
+
+// bf16 GEMM on the cluster split-K kernel; 1 (nothing launched) when the other kernels are expected to be faster.
+static int run_cluster(const FusedArgs &a) {
+    ClusterGemmParams p;
+    memset(&p, 0, sizeof(p));
+    p.M = a.M;
+    p.k_blocks = a.K / 64;
+    p.epi = a.epi;
+    p.num_segs = a.num_w;
+    int tiles = 0;
+    double n_rows = 0.0;
+    const bool silu = a.epi == EPI_SILU_GATE;
+    for (int i = 0; i < a.num_w; ++i) {
+        p.seg_rows[i] = a.n_bf16[i];
+        p.seg_tiles[i] = silu ? (a.n_bf16[i] + 63) / 64 : (a.n_bf16[i] + 127) / 128;
+        if (i == 0 || !silu) tiles += p.seg_tiles[i];
+        n_rows += a.n_bf16[i];
+    }
+    // the single-CTA kernel: about 0.25 us per 64-wide k block of a 128 x 128 tile, one tile per SM and round
+    const double cluster_ns = choose_cluster_gemm(p, tiles);
+    const double rounds = ((a.M + 127) / 128 * (silu ? 2 * ((a.n_bf16[0] + 127) / 128) : tiles) + num_sms() - 1) / num_sms();
+    if (cluster_ns == 0.0 || cluster_ns > 3000.0 + 250.0 * p.k_blocks * rounds) return 1;
+    for (int i = 0; i < a.num_w; ++i)
+        if (!make_tmap(&p.tm_w[i], a.w_bf16[i], CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)a.K, (uint64_t)a.n_bf16[i],
+                       (uint64_t)a.K * 2, 64, silu ? 64 : 128, true))
+            return -1;
+    if (!make_tmap(&p.tm_x, a.x, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)a.K, (uint64_t)a.M, (uint64_t)a.ldx * 2, 64,
+                   (uint32_t)p.n_tok, true))
+        return -1;
+    p.out = a.out;
+    p.residual = a.residual;
+    p.bias = a.bias;
+    p.ldo = a.ldo;
+    p.early_weights = a.const_weights && pdl_enabled() ? 1 : 0;
+    p.status = device_status_word();
+    profile_bracket_begin(2.0 * a.M * n_rows * a.K, 2.0 * n_rows * a.K + 2.0 * a.M * (a.K + total_out_cols(a)) +
+                                                        (a.epi == EPI_RESIDUAL ? 2.0 * a.M * total_out_cols(a) : 0.0));
+    if (launch_cluster_gemm(p, g_stream) != cudaSuccess) return -1;
+    profile_bracket_end();
+    ++g_launches;
+    return 0;
+}
+
 static int run_fused(const FusedArgs &a) {
     if (a.M <= 0 || a.K <= 0) return -1;
     if (a.mode != GEMM_BF16) {
@@ -628,7 +685,7 @@ static int run_fused(const FusedArgs &a) {
         return run_simt(a);
     }
 
-    // A handful of rows: the few-row kernel reads the packed weights as they are.  W4A16 takes it up to its 32 rows.  A
+    // A handful of rows: the few-row kernel reads the packed weights as they are.  W4A16 takes it up to its 16 rows.  A
     // single W4A4 linear does up to 8 (every CTA quantises the rows for itself); fused W4A4 projections and quantised
     // hand-overs, the parts of a chain, stay on the block-scaled MMA whose bits they share with the resident kernel.
     if (skinny_eligible(a)) return run_skinny(a);
@@ -651,6 +708,7 @@ static int run_fused(const FusedArgs &a) {
                 b.n_bf16[i] = a.w[i].N;
             }
             b.w = nullptr;
+            b.const_weights = true;         // the copy is made by an ordinary launch, which ends before anything behind it starts
             return run_fused(b);
         }
     }
@@ -676,6 +734,11 @@ static int run_fused(const FusedArgs &a) {
         }
         b.w = nullptr;
         return run_fused(b);
+    }
+
+    if (a.mode == GEMM_BF16 && a.q_out == nullptr && a.pre == nullptr && route_rows(a) <= cluster_gemm_rows()) {
+        const int rc = run_cluster(a);
+        if (rc <= 0) return rc;
     }
 
     const int dev = current_device();
@@ -1009,7 +1072,7 @@ int fp4_linear_w4a16_silu_quantized(uint8_t *q_out, uint8_t *q_out_sf, float q_o
 // residual row pitch ldo).  x row pitch ldx, out row pitch ldo.  Returns 0, or -1 when the shape cannot run on
 // the tensor-core path (K % 64, 16-byte alignment).
 int bf16_linear_ex(uint16_t *out, int ldo, const uint16_t *x, int ldx, const uint16_t *const *w, const int *n, int num_w,
-                   const uint16_t *bias, int epi, const uint16_t *residual, int M, int K) {
+                   const uint16_t *bias, int epi, const uint16_t *residual, int M, int K, bool const_weights) {
     if (out == nullptr || x == nullptr || w == nullptr || n == nullptr || num_w < 1 || num_w > kMaxSegments || M <= 0 || K <= 0)
         return -1;
     if (epi == EPI_RESIDUAL && residual == nullptr) return -1;
@@ -1031,6 +1094,7 @@ int bf16_linear_ex(uint16_t *out, int ldo, const uint16_t *x, int ldx, const uin
     a.residual = (const __nv_bfloat16 *)residual;
     a.M = M;
     a.K = K;
+    a.const_weights = const_weights;
     if (ldo < total_out_cols(a) || ldx < K) return -1;
     if (!tensor_core_eligible(a)) return -1;
     return run_fused(a);
@@ -1135,7 +1199,7 @@ extern "C" void bf16_linear_gelu(void *handle, uint16_t *out, const uint16_t *x,
     if (M <= 0 || N <= 0 || K <= 0) return;
     const uint16_t *ws[1] = {w};
     const int ns[1] = {N};
-    GLMASR_CHECK(bf16_linear_ex(out, N, x, K, ws, ns, 1, bias, EPI_GELU, nullptr, M, K) == 0,
+    GLMASR_CHECK(bf16_linear_ex(out, N, x, K, ws, ns, 1, bias, EPI_GELU, nullptr, M, K, false) == 0,
                  "bf16_linear_gelu: unsupported shape or alignment (M=%d N=%d K=%d)", M, N, K);
     GLMASR_CUDA_CHECK(cudaGetLastError());
 }

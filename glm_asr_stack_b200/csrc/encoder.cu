@@ -35,7 +35,7 @@
 namespace glmasr {
 
 int bf16_linear_ex(uint16_t *out, int ldo, const uint16_t *x, int ldx, const uint16_t *const *w, const int *n, int num_w,
-                   const uint16_t *bias, int epi, const uint16_t *residual, int M, int K);   // api.cu
+                   const uint16_t *bias, int epi, const uint16_t *residual, int M, int K, bool const_weights);   // api.cu
 
 // private workspace slots of this file
 enum : int { WS_E_NORM = 38, WS_E_QKV = 39, WS_E_FFN = 40, WS_E_POS = 41, WS_E_META = 42, WS_E_COL = 43, WS_E_CONV1 = 44,
@@ -166,7 +166,7 @@ __global__ void encoder_rope_kernel(__nv_bfloat16 *q, __nv_bfloat16 *k, const fl
     if (idx >= total_rows * num_heads * kRotHalf) return;
     const int d = idx % kRotHalf, rh = idx / kRotHalf;
     const int head = rh % num_heads, row = rh / num_heads;
-    const int pos = row_pos[row];
+    const int pos = (int)min((unsigned)row_pos[row], (unsigned)(kRopeTablePos - 1));     // a row of no sequence has no position
     const float c = cos_t[pos * kRotHalf + d], s = sin_t[pos * kRotHalf + d];
     if (q != nullptr) {
         __nv_bfloat16 *p = q + (size_t)row * q_stride + head * head_dim;
@@ -193,7 +193,7 @@ __global__ void __launch_bounds__(256) encoder_rope_vec_kernel(__nv_bfloat16 *q,
     if (idx >= total_rows * num_heads * 2) return;
     const int d0 = (idx & 1) * 8, rh = idx >> 1;
     const int head = rh % num_heads, row = rh / num_heads;
-    const int pos = row_pos[row];
+    const int pos = (int)min((unsigned)row_pos[row], (unsigned)(kRopeTablePos - 1));     // a row of no sequence has no position
     float c[8], s[8];
     {
         const float4 *cp = reinterpret_cast<const float4 *>(cos_t + pos * kRotHalf + d0);
@@ -503,7 +503,7 @@ static int gemm(uint16_t *out, int ldo, const uint16_t *x, int ldx, const uint16
                 const uint16_t *residual, int M, int K) {
     const uint16_t *ws[1] = {w};
     const int ns[1] = {N};
-    return bf16_linear_ex(out, ldo, x, ldx, ws, ns, 1, bias, epi, residual, M, K);
+    return bf16_linear_ex(out, ldo, x, ldx, ws, ns, 1, bias, epi, residual, M, K, true);
 }
 
 // The 32 layers and the final norm, in place on hidden [total_rows, H]; d_meta = device {offsets[num_seqs], lens[num_seqs]}.
@@ -526,7 +526,7 @@ static void encoder_layers(const glmasr_WeightStore *ws, const glmasr_ModelConfi
                          (const __nv_bfloat16 *)W.ln1_b, 1e-5f, M, H, st);
         const uint16_t *w3[3] = {W.q_w, W.k_w, W.v_w};
         const int n3[3] = {H, H, H};
-        GLMASR_CHECK(bf16_linear_ex(qkv, 3 * H, nrm, H, w3, n3, 3, W.qkv_bias, EPI_STORE, nullptr, M, H) == 0,
+        GLMASR_CHECK(bf16_linear_ex(qkv, 3 * H, nrm, H, w3, n3, 3, W.qkv_bias, EPI_STORE, nullptr, M, H, true) == 0,
                      "encoder q|k|v projection failed (rows %d)", M);
         launch_encoder_rope((__nv_bfloat16 *)qkv, (__nv_bfloat16 *)qkv + H, row_pos, M, NH, HD, 3 * H, 3 * H, st);
         const bool ok = launch_prefill_attention((__nv_bfloat16 *)nrm, H, (const __nv_bfloat16 *)qkv, 3 * H,

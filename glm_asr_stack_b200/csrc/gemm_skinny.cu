@@ -1,6 +1,6 @@
 // W4A16 / W4A4 linear for a handful of rows (decode of a few sequences).
 //
-// With M <= 32 rows the tcgen05 kernels leave most of the chip idle: a 2048-column projection has sixteen 128-wide
+// With M <= 16 rows the tcgen05 kernels leave most of the chip idle: a 2048-column projection has sixteen 128-wide
 // tiles, and each of those CTAs pulls its whole K range through one ring at the ~100 GB/s one SM gets (down projection,
 // K = 6144: 27 us; a decode step of one sequence took 2.56 ms, 0.06 of the rate of the bytes it has to read).  Here the
 // weights are the MMA's 16-row operand and the tokens its 8-column operand (mma.sync m16n8k16: 128 token lanes of a
@@ -20,6 +20,8 @@
 //     multiplies the fp32 sums.  W4A4 rounds x through the activation quantiser instead: e2m1 * e4m3 is exact in bf16
 //     and the products are exact in fp32, so the result is the block-scaled MMA's up to the order of the sum;
 //   * the eight partial sums meet in shared memory, fixed order.
+// From 17 rows the tokens' operand no longer fits the registers beside the accumulators and the bf16 copies on the cluster
+// GEMM are faster (19 sequences: 1.96 against 2.33 ms a step).
 // Bound: instruction issue of the dequantisation (five instructions per two weights; 1.8 us for gate|up) and the fixed
 // latencies of a launch in a dependent chain, with the 28 MB of a layer's weights streamed underneath.
 #include "gemm_skinny.cuh"
@@ -35,10 +37,10 @@ namespace glmasr {
 
 static constexpr int kWarpsSk = 8;
 static constexpr int kThreadsSk = kWarpsSk * 32;
-static constexpr int kSmemHeader = 1280;            // barriers, abort word, sums of squares [8][32]
+static constexpr int kSmemHeader = 1280;            // barriers, abort word, sums of squares [8][16]
 static constexpr int kSmemWeights = 150 * 1024;     // most that weight slots may take
 
-__host__ __device__ constexpr int sk_tiles_per_pass(int nt) { return nt == 1 ? 6 : (nt == 2 ? 4 : 2); }
+__host__ __device__ constexpr int sk_tiles_per_pass(int nt) { return nt == 1 ? 6 : 4; }
 __host__ __device__ inline int sk_slot_bytes(int K) { return 16 * (K / 2 + 16) + 16 * (K / 16 + 16); }
 
 __device__ __forceinline__ uint32_t lds16_sk(uint32_t a) {
@@ -360,7 +362,7 @@ cudaError_t launch_skinny_linear(SkinnyParams p, int num_sms, cudaStream_t st) {
     p.units = rows / 16;
     p.units_per_cta = (p.units + num_sms - 1) / num_sms;
     const int unit_bytes = mt * sk_slot_bytes(p.K);
-    const int nt = p.M <= 8 ? 1 : (p.M <= 16 ? 2 : 4);
+    const int nt = p.M <= 8 ? 1 : 2;
     const int per_pass = sk_tiles_per_pass(nt) / mt;         // units accumulated at a time
     if (p.units_per_cta * unit_bytes <= kSmemWeights) {
         p.groups = 1;
@@ -375,11 +377,7 @@ cudaError_t launch_skinny_linear(SkinnyParams p, int num_sms, cudaStream_t st) {
     p.pass_tiles = sk_tiles_per_pass(nt) < p.units_per_group * mt ? sk_tiles_per_pass(nt) : p.units_per_group * mt;
     const size_t smem = kSmemHeader + (size_t)p.groups * p.units_per_group * unit_bytes +
                         (size_t)kWarpsSk * p.pass_tiles * 16 * nt * 8 * sizeof(float);
-    switch (nt) {
-        case 1: return launch_nt<1>(p, grid, smem, st);
-        case 2: return launch_nt<2>(p, grid, smem, st);
-        default: return launch_nt<4>(p, grid, smem, st);
-    }
+    return nt == 1 ? launch_nt<1>(p, grid, smem, st) : launch_nt<2>(p, grid, smem, st);
 }
 
 }  // namespace glmasr

@@ -1,4 +1,4 @@
-// Few-row FP4 linear (gemm_skinny.cu): out[M, sum N_s] = epilogue(x[M, K] * concat_s(W_s[N_s, K])^T) for M <= 32,
+// Few-row FP4 linear (gemm_skinny.cu): out[M, sum N_s] = epilogue(x[M, K] * concat_s(W_s[N_s, K])^T) for M <= 16,
 // reading the packed e2m1 weights and their e4m3 scales as stored.
 #pragma once
 #include <cuda_bf16.h>
@@ -7,7 +7,7 @@
 
 namespace glmasr {
 
-static constexpr int kSkinnyMaxRows = 32;
+static constexpr int kSkinnyMaxRows = 16;
 
 struct SkinnyParams {
     const __nv_bfloat16 *x;             // [M, K], row pitch ldx (multiple of 8 elements, 16-byte aligned)

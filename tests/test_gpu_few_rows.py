@@ -1,5 +1,5 @@
-"""The few-row FP4 linear (1 to 32 rows of W4A16, 1 to 8 of a single W4A4 linear) at the edges of its token tiles (8, 16, 32),
-of its 16-row units and of its chunks of K, against the float32 oracles.  Tolerance: one bf16 rounding of the result
+"""The few-row FP4 linear (1 to 16 rows of W4A16, 1 to 8 of a single W4A4 linear) at the edges of its token tiles (8, 16),
+of its 16-row units and of its chunks of K, and the first sizes of the bf16 route behind it, against the float32 oracles.  Tolerance: one bf16 rounding of the result
 (2^-9) and the order of a float32 sum of at most 8192 exact products, the bar every other route is held to."""
 import numpy as np
 import pytest
@@ -66,3 +66,19 @@ def test_scale_codes(ops):
         xb = (x.view(np.uint32) >> 16).astype(np.uint16)
         out = ops.fp4_linear(to_dev_bf16(xb), to_dev_u8(packed), to_dev_u8(scales), 1.0)
         assert o.rel_err(bits_of(out), o.linear_o1(xb, packed, scales, 1.0)) <= REL_TOL_TIGHT
+
+
+@pytest.mark.parametrize("M", [17, 64, 65, 173, 257, 512])
+@pytest.mark.parametrize("N,K", [(136, 64), (1288, 5120), (2048, 1984)])
+def test_cluster_split_k(ops, M, N, K):
+    """bf16 linear of 17 to 512 rows (K cut over a cluster where that pays), ragged rows, columns and K shares: plain with
+    bias, GELU, and the same sum against float32.  REL_TOL_TIGHT: one bf16 rounding and the order of the float32 sum."""
+    gen = torch.Generator(device="cuda").manual_seed(M + N)
+    x, w = (torch.randn(s, generator=gen, device="cuda").to(torch.bfloat16) for s in ((M, K), (N, K)))
+    b = torch.randn(N, generator=gen, device="cuda").to(torch.bfloat16)
+    want = x.double() @ w.double().T + b.double()
+    got = ops.bf16_linear(x, w, b).double()
+    assert float((got - want).norm() / want.norm()) <= REL_TOL_TIGHT
+    want = torch.nn.functional.gelu(want, approximate="tanh")
+    got = ops.bf16_linear_gelu(x, w, b).double()
+    assert float((got - want).norm() / want.norm()) <= REL_TOL_TIGHT
