@@ -77,6 +77,9 @@ bool launch_prefill_attention(__nv_bfloat16 *out, int ldo, const __nv_bfloat16 *
                               int head_dim, bool causal, cudaStream_t st, uint8_t *q_packed = nullptr,
                               uint8_t *q_sf = nullptr, float q_input_scale = 0.0f);
 // The tcgen05 kernel behind it (prefill_attention_umma.cu); false = shape or alignment not covered.
+bool launch_attention64_umma(__nv_bfloat16 *out, int ldo, const __nv_bfloat16 *q, int ldq, const __nv_bfloat16 *k, int ldk,
+                             const __nv_bfloat16 *v, int ldv, const int *seq_offsets, const int *seq_lens, int num_seqs,
+                             int max_seq_len, int total_tokens, int num_q_heads, int num_kv_heads, bool causal, cudaStream_t st);
 bool launch_prefill_attention_umma(__nv_bfloat16 *out, int ldo, const __nv_bfloat16 *q, int ldq, const __nv_bfloat16 *k,
                                    int ldk, const __nv_bfloat16 *v, int ldv, const int *seq_offsets, const int *seq_lens,
                                    int num_seqs, int max_seq_len, int total_tokens, int num_q_heads, int num_kv_heads,

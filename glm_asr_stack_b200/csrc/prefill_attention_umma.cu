@@ -6,7 +6,7 @@
 // Persistent CTAs (two per SM) take work items = 128 queries of one (sequence, q head), longest first; the
 // keys of an item are walked in steps of 64:
 //   warp 0      TMA producer: Q once per item (two 128-row x 64-dim boxes), then per step the K tile (two 64-row
-//               boxes) and the V^T tile (128 dims x 64 keys) into two-stage rings, 128-byte swizzle;
+//               boxes) and the V tile (the same two boxes) into two-stage rings, 128-byte swizzle;
 //   warp 1      MMA issuer: S_j = Q K_j^T (M 128, N 64, K 128) into one of two TMEM score buffers, and
 //               O += P_j V_j (M 128, N 128, K 64) into the TMEM output accumulator; S_{j+1} is issued
 //               before P_j V_j so that the soft-max of step j+1 never waits for the second product;
@@ -17,10 +17,8 @@
 //               against -- the final division by the row sum uses the same reference value, so the
 //               result is that of the ordinary online soft-max up to rounding.
 // 112 KB of shared memory and 256 TMEM columns per CTA: two CTAs per SM, one's soft-max under the
-// other's MMAs.  V is consumed as V^T (keys contiguous) so that both products take K-major
-// operands: transpose_v_kernel writes V^T for every kv head into a private workspace first, each
-// sequence starting at a multiple of 64 columns and zero-filled to the next multiple (10 MB per
-// layer at 10000 tokens, a few microseconds).
+// other's MMAs.  V is read as it lies in memory, [key][dim]: the second product's B operand is MN-major (as V^T it needed a
+// transposing launch in front of every layer's attention, 7 us at 10000 tokens and 4.5 us at 173).
 // Every wait is bounded (status ST_TIMEOUT_ATTENTION); nothing here loads with cluster-wide delivery.
 #include <cuda_bf16.h>
 #include <math.h>
@@ -45,20 +43,18 @@ constexpr int TMEM_COLS = 256;                // S0 [0,64), S1 [64,128), O [128,
 constexpr int THREADS = 192;
 constexpr float kRescaleThreshold = 8.0f;     // log2 units
 
-// Shared-memory layout for one head_dim (64: the audio encoder, 128: the decoder).  Rows of Q and K are cut
-// into 64-dim boxes of 128 bytes (the widest box the 128-byte swizzle takes).
-template <int HD>
-struct Geo {
-    static_assert(HD == 64 || HD == 128, "head_dim 64 or 128");
-    static constexpr int NB = HD / 64;                 // 64-dim boxes per Q / K row
+constexpr int HD = 128;
+// Shared-memory layout.  Rows of Q, K and V are cut into 64-dim boxes of 128 bytes (the widest box the 128-byte swizzle takes).
+struct G {
+    static constexpr int NB = HD / 64;                 // 64-dim boxes per row
     static constexpr int Q_BYTES = NB * 128 * 128;
     static constexpr int K_BYTES = NB * KT * 128;
-    static constexpr int V_BYTES = HD * 128;           // V^T: head_dim dims x 64 keys
+    static constexpr int V_BYTES = NB * KT * 128;
     static constexpr int OFF_Q = 0;
     static constexpr int OFF_K = OFF_Q + Q_BYTES;
     static constexpr int OFF_V = OFF_K + 2 * K_BYTES;
     static constexpr int OFF_P = OFF_V + 2 * V_BYTES;
-    static constexpr int OFF_BAR = OFF_P + P_BYTES;    // tiles (112 KB / 64 KB), then barriers
+    static constexpr int OFF_BAR = OFF_P + P_BYTES;    // 112 KB of tiles, then barriers
     static constexpr int OFF_OS_TABLE = OFF_BAR + 256; // 128 floats: the quantiser's second division, one entry per scale byte
     static constexpr int SMEM_BYTES = OFF_OS_TABLE + 512;
 };
@@ -67,12 +63,11 @@ enum : int { B_QFULL = 0, B_KFULL = 1, B_KEMPTY = 3, B_VFULL = 5, B_VEMPTY = 7, 
              B_PVDONE = 14, B_QEMPTY = 15, B_OFREE = 16 };
 
 struct AttnParams {
-    CUtensorMap tm_q, tm_k, tm_vt;
+    CUtensorMap tm_q, tm_k, tm_v;
     __nv_bfloat16 *out;
     const int *seq_offsets;
     const int *seq_lens;          // NULL: seq_offsets is cumulative (num_seqs + 1 entries)
     int *status;
-    const int *vt_col;            // first V^T column of every sequence (written by transpose_v_kernel)
     unsigned long long *dbg;      // experiment builds (-DGLMASR_EXPERIMENTS): 8 cycle sums per CTA (soft-max warp 2), else NULL
     int dbg_no_store;             // experiment builds: leave the result stores out
     int ldo, num_q_heads, num_seqs, group, q_tiles, total_items, causal;
@@ -87,14 +82,6 @@ struct AttnParams {
 __device__ __forceinline__ int seq_len_of(const int *offs, const int *lens, int s) {
     return lens != nullptr ? lens[s] : offs[s + 1] - offs[s];
 }
-// First V^T column of sequence `seq`: the lengths before it, each rounded up to 64.
-__device__ __forceinline__ int padded_column_of(const int *offs, const int *lens, int seq, int lane) {
-    int col = 0;
-    for (int s = lane; s < seq; s += 32) col += (seq_len_of(offs, lens, s) + 63) & ~63;
-#pragma unroll
-    for (int d = 16; d > 0; d >>= 1) col += __shfl_xor_sync(0xFFFFFFFFu, col, d);
-    return col;
-}
 __device__ __forceinline__ float ex2(float x) {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -103,63 +90,6 @@ __device__ __forceinline__ float ex2(float x) {
 __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
     const __nv_bfloat162 b = __floats2bfloat162_rn(lo, hi);
     return *reinterpret_cast<const uint32_t *>(&b);
-}
-
-// vt[(h * HD + d) * vt_cols + col(seq) + t] = v[(off(seq) + t) * ldv + h * HD + d], zero for t >= len
-// up to the next multiple of 64.  grid = (64-token tiles, kv heads, sequences).
-template <int HD>
-__global__ void __launch_bounds__(256) transpose_v_kernel(__nv_bfloat16 *__restrict__ vt, int vt_cols,
-                                                         const __nv_bfloat16 *__restrict__ v, int ldv,
-                                                         const int *__restrict__ seq_offsets,
-                                                         const int *__restrict__ seq_lens, int *__restrict__ vt_col,
-                                                         int *status) {
-    __shared__ uint32_t tile[64][HD / 2 + 1];  // [token][dim pair], odd pitch
-    __shared__ int s_col;
-    pdl_launch_dependents();
-    pdl_wait();
-    const int seq = blockIdx.z, h = blockIdx.y, t0 = blockIdx.x * 64;
-    const int off = seq_offsets[seq];
-    const int len = seq_len_of(seq_offsets, seq_lens, seq);
-    if (t0 >= len) return;
-    if (threadIdx.x < 32) {
-        const int col = padded_column_of(seq_offsets, seq_lens, seq, threadIdx.x);
-        if (threadIdx.x == 0) {
-            s_col = col;
-            if (blockIdx.x == 0 && blockIdx.y == 0) vt_col[seq] = col;
-        }
-    }
-    constexpr int CH = HD / 8;                  // 16-byte chunks (8 dims) per token row
-#pragma unroll
-    for (int i = 0; i < 64 * CH / 256; ++i) {
-        const int idx = threadIdx.x + i * 256;
-        const int r = idx / CH, c = idx % CH;          // token row, 16-byte chunk (8 dims)
-        uint4 val = make_uint4(0u, 0u, 0u, 0u);
-        if (t0 + r < len) val = *reinterpret_cast<const uint4 *>(v + (size_t)(off + t0 + r) * ldv + (size_t)h * HD + c * 8);
-        tile[r][c * 4 + 0] = val.x;
-        tile[r][c * 4 + 1] = val.y;
-        tile[r][c * 4 + 2] = val.z;
-        tile[r][c * 4 + 3] = val.w;
-    }
-    __syncthreads();
-    const int col = s_col;
-    if (col + t0 + 64 > vt_cols) {              // the workspace was sized from the caller's token count
-        if (threadIdx.x == 0 && status != nullptr) atomicCAS(status, 0, ST_BAD_LAYOUT);
-        return;
-    }
-#pragma unroll
-    for (int i = 0; i < HD * 8 / 256; ++i) {
-        const int idx = threadIdx.x + i * 256;
-        const int d = idx >> 3, c = idx & 7;           // dim row, 16-byte chunk (8 tokens)
-        uint32_t w[4];
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const uint32_t a = tile[c * 8 + 2 * e][d >> 1], b = tile[c * 8 + 2 * e + 1][d >> 1];
-            const uint32_t lo = (d & 1) ? (a >> 16) : (a & 0xFFFFu);
-            const uint32_t hi = (d & 1) ? (b >> 16) : (b & 0xFFFFu);
-            w[e] = lo | (hi << 16);
-        }
-        *reinterpret_cast<uint4 *>(vt + (size_t)(h * HD + d) * vt_cols + col + t0 + c * 8) = make_uint4(w[0], w[1], w[2], w[3]);
-    }
 }
 
 // Work item = (128-query tile, sequence, q head).  Items are numbered with the last (longest, when causal)
@@ -183,9 +113,7 @@ __device__ __forceinline__ bool decode_item(const AttnParams &p, int item, ItemI
     return true;
 }
 
-template <int HD>
 __global__ void __launch_bounds__(THREADS, 2) prefill_attention_umma_kernel(const __grid_constant__ AttnParams p) {
-    using G = Geo<HD>;
     constexpr int OFF_Q = G::OFF_Q, OFF_K = G::OFF_K, OFF_V = G::OFF_V, OFF_P = G::OFF_P, OFF_BAR = G::OFF_BAR;
     constexpr int OFF_OS_TABLE = G::OFF_OS_TABLE, Q_BYTES = G::Q_BYTES, K_BYTES = G::K_BYTES, V_BYTES = G::V_BYTES;
     extern __shared__ __align__(1024) uint8_t smem[];
@@ -218,7 +146,7 @@ __global__ void __launch_bounds__(THREADS, 2) prefill_attention_umma_kernel(cons
         fence_mbar_init();
         tma_prefetch_desc(&p.tm_q);
         tma_prefetch_desc(&p.tm_k);
-        tma_prefetch_desc(&p.tm_vt);
+        tma_prefetch_desc(&p.tm_v);
     }
     if (warp == 1) {
         tmem_alloc(smem_u32((const void *)tmem_slot), TMEM_COLS);
@@ -241,7 +169,6 @@ __global__ void __launch_bounds__(THREADS, 2) prefill_attention_umma_kernel(cons
             ItemInfo it;
             if (!decode_item(p, item, it)) continue;
             const int kv_head = it.head / p.group;
-            const int col = p.vt_col[it.seq];
             if (!mbar_wait_warp(bar(B_QEMPTY), (qi & 1u) ^ 1u, abort_word, ST_TIMEOUT_ATTENTION)) break;
             if (leader) {
                 mbar_expect_tx(bar(B_QFULL), Q_BYTES);
@@ -264,7 +191,10 @@ __global__ void __launch_bounds__(THREADS, 2) prefill_attention_umma_kernel(cons
                 if (!mbar_wait_warp(bar(B_VEMPTY + s), ph ^ 1u, abort_word, ST_TIMEOUT_ATTENTION)) { ok = false; break; }
                 if (leader) {
                     mbar_expect_tx(bar(B_VFULL + s), V_BYTES);
-                    tma_load_2d(sbase + OFF_V + (uint32_t)s * V_BYTES, &p.tm_vt, bar(B_VFULL + s), col + j * KT, kv_head * HD);
+#pragma unroll
+                    for (int b = 0; b < G::NB; ++b)
+                        tma_load_2d(sbase + OFF_V + (uint32_t)s * V_BYTES + b * (V_BYTES / G::NB), &p.tm_v, bar(B_VFULL + s),
+                                    kv_head * HD + 64 * b, it.off + j * KT);
                 }
             }
         }
@@ -272,7 +202,7 @@ __global__ void __launch_bounds__(THREADS, 2) prefill_attention_umma_kernel(cons
         // ================================ MMA issuer ==================================
         const bool leader = elect_one();
         constexpr uint32_t idesc_s = idesc_bf16(128, KT);
-        constexpr uint32_t idesc_o = idesc_bf16(128, HD);
+        constexpr uint32_t idesc_o = idesc_bf16(128, HD) | kIdescBMnMajor;
         const uint32_t t_o = tmem_base + 128;
         uint32_t ks = 0, kp = 0, qi = 0;        // S products issued, P V products issued, items started
         bool ok = true;
@@ -312,10 +242,10 @@ __global__ void __launch_bounds__(THREADS, 2) prefill_attention_umma_kernel(cons
                     tc_fence_after();
                     if (leader) {
                         const uint64_t adesc0 = smem_desc_sw128(sbase + OFF_P);
-                        const uint64_t bdesc0 = smem_desc_sw128(sbase + OFF_V + (uint32_t)s * V_BYTES);
+                        const uint64_t bdesc0 = smem_desc_sw128_mn(sbase + OFF_V + (uint32_t)s * V_BYTES, V_BYTES / G::NB);
 #pragma unroll
                         for (int k = 0; k < 4; ++k)
-                            umma_bf16(t_o, adesc0 + (uint64_t)((k * 32) >> 4), bdesc0 + (uint64_t)((k * 32) >> 4), idesc_o,
+                            umma_bf16(t_o, adesc0 + (uint64_t)((k * 32) >> 4), bdesc0 + (uint64_t)((k * 2048) >> 4), idesc_o,
                                       (j > 1 || k > 0) ? 1u : 0u);
                         umma_commit(bar(B_VEMPTY + s));
                         umma_commit(bar(B_PVDONE));
@@ -431,6 +361,16 @@ __global__ void __launch_bounds__(THREADS, 2) prefill_attention_umma_kernel(cons
                                  "r"(pk[4 * ch + 2]), "r"(pk[4 * ch + 3])
                                  : "memory");
                 }
+                // keys past the sequence's end weigh nothing, but the rows behind it may hold anything (another sequence, or
+                // memory nobody wrote): 0 * NaN must not reach the sum
+                const int v_rows = len - j * KT;
+                if (v_rows < KT) {
+                    if (!mbar_wait_warp(bar(B_VFULL + b), (sc >> 1) & 1u, abort_word, ST_TIMEOUT_ATTENTION)) { ok = false; break; }
+                    for (int c = v_rows * 8 + row; c < KT * 8; c += 128)
+#pragma unroll
+                        for (int h = 0; h < G::NB; ++h)
+                            asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(sbase + OFF_V + (uint32_t)b * V_BYTES + (uint32_t)(h * (V_BYTES / G::NB) + c * 16)), "r"(0) : "memory");
+                }
                 fence_proxy_async_smem();
                 tc_fence_before();
                 mbar_arrive(bar(B_PFULL));
@@ -448,7 +388,7 @@ __global__ void __launch_bounds__(THREADS, 2) prefill_attention_umma_kernel(cons
             // cover whole 128-byte (bf16) or 64-byte (quantised) row segments instead of 16 bytes per row.
             const int wrow0 = quad * 32;                               // first tile row of this warp
             const uint32_t stage = sbase + OFF_P + (uint32_t)wrow0 * 128u;
-            if (HD != 128 || p.q_packed == nullptr) {
+            if (p.q_packed == nullptr) {
 #pragma unroll 1
                 for (int half = 0; half < HD / 64; ++half) {
 #pragma unroll
@@ -485,7 +425,7 @@ __global__ void __launch_bounds__(THREADS, 2) prefill_attention_umma_kernel(cons
                     }
                     __syncwarp();
                 }
-            } else if constexpr (HD == 128) {
+            } else {
                 // a row of one head is eight 16-element blocks of the quantiser: 64 packed bytes, 8 scale bytes
                 uint32_t sf_lo = 0u, sf_hi = 0u;
 #pragma unroll 1
@@ -580,30 +520,25 @@ bool launch_prefill_attention_umma(__nv_bfloat16 *out, int ldo, const __nv_bfloa
         return false;
     if ((head_dim != 128 && head_dim != 64) || num_kv_heads <= 0 || num_q_heads % num_kv_heads != 0 || total_tokens <= 0) return false;
     if (head_dim != 128 && q_packed != nullptr) return false;          // the quantising epilogue exists for head_dim 128 only
-    const int HD = head_dim;
     if ((ldq % 8) != 0 || (ldo % 8) != 0 || (ldk % 8) != 0 || (ldv % 8) != 0) return false;
     if ((((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)out) & 15) != 0) return false;
-    if (ldq < num_q_heads * HD || ldk < num_kv_heads * HD) return false;
+    if (ldq < num_q_heads * head_dim || ldk < num_kv_heads * head_dim || ldv < num_kv_heads * head_dim) return false;
+    if (head_dim == 64)
+        return launch_attention64_umma(out, ldo, q, ldq, k, ldk, v, ldv, seq_offsets, seq_lens, num_seqs, max_seq_len, total_tokens,
+                                       num_q_heads, num_kv_heads, causal, st);
     static bool configured = false;
     if (!configured) {
-        if (cudaFuncSetAttribute(prefill_attention_umma_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, Geo<128>::SMEM_BYTES) !=
-                cudaSuccess ||
-            cudaFuncSetAttribute(prefill_attention_umma_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, Geo<64>::SMEM_BYTES) !=
-                cudaSuccess)
+        if (cudaFuncSetAttribute(prefill_attention_umma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, G::SMEM_BYTES) != cudaSuccess)
             return false;
-        cudaFuncSetAttribute(prefill_attention_umma_kernel<128>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                             (int)cudaSharedmemCarveoutMaxShared);
-        cudaFuncSetAttribute(prefill_attention_umma_kernel<64>, cudaFuncAttributePreferredSharedMemoryCarveout,
+        cudaFuncSetAttribute(prefill_attention_umma_kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
                              (int)cudaSharedmemCarveoutMaxShared);
         configured = true;
     }
-    const int vt_cols = (total_tokens + 64 * num_seqs + 63) & ~63;
-    __nv_bfloat16 *vt = (__nv_bfloat16 *)workspace_slot(WS_ATTN_VT, (size_t)num_kv_heads * HD * (size_t)vt_cols * 2);
     AttnParams p;
     memset(&p, 0, sizeof(p));
     if (!make_bf16_tmap_sw128(&p.tm_q, q, (uint64_t)num_q_heads * HD, (uint64_t)total_tokens, (uint64_t)ldq * 2, 64, 128)) return false;
     if (!make_bf16_tmap_sw128(&p.tm_k, k, (uint64_t)num_kv_heads * HD, (uint64_t)total_tokens, (uint64_t)ldk * 2, 64, KT)) return false;
-    if (!make_bf16_tmap_sw128(&p.tm_vt, vt, (uint64_t)vt_cols, (uint64_t)num_kv_heads * HD, (uint64_t)vt_cols * 2, 64, HD)) return false;
+    if (!make_bf16_tmap_sw128(&p.tm_v, v, (uint64_t)num_kv_heads * HD, (uint64_t)total_tokens, (uint64_t)ldv * 2, 64, KT)) return false;
     p.out = out;
     p.seq_offsets = seq_offsets;
     p.seq_lens = seq_lens;
@@ -614,8 +549,6 @@ bool launch_prefill_attention_umma(__nv_bfloat16 *out, int ldo, const __nv_bfloa
     p.q_tiles = (max_seq_len + QT - 1) / QT;
     p.num_seqs = num_seqs;
     p.total_items = p.q_tiles * num_q_heads * num_seqs;
-    int *vt_col = (int *)workspace_slot(WS_ATTN_VT_COL, (size_t)num_seqs * sizeof(int));
-    p.vt_col = vt_col;
     p.causal = causal ? 1 : 0;
     p.scale_log2 = 1.4426950408889634f / sqrtf((float)head_dim);
     p.q_packed = q_packed;
@@ -624,12 +557,6 @@ bool launch_prefill_attention_umma(__nv_bfloat16 *out, int ldo, const __nv_bfloa
     p.q_sf_chunks = num_q_heads * 2;
     p.q_inv_in = q_packed != nullptr ? 1.0f / q_input_scale : 0.0f;
 
-    const dim3 tgrid((max_seq_len + 63) / 64, num_kv_heads, num_seqs);
-    if (HD == 128)
-        launch_chained(transpose_v_kernel<128>, tgrid, dim3(256), (size_t)0, st, vt, vt_cols, v, ldv, seq_offsets, seq_lens, vt_col, p.status);
-    else
-        launch_chained(transpose_v_kernel<64>, tgrid, dim3(256), (size_t)0, st, vt, vt_cols, v, ldv, seq_offsets, seq_lens, vt_col, p.status);
-    note_launches(1);
     static int num_sms = 0;
     if (num_sms == 0) {
         int dev = 0;
@@ -649,10 +576,7 @@ bool launch_prefill_attention_umma(__nv_bfloat16 *out, int ldo, const __nv_bfloa
         cudaMemsetAsync(p.dbg, 0, (size_t)grid.x * 8 * sizeof(unsigned long long), st);
     }
 #endif
-    if (HD == 128)
-        launch_chained(prefill_attention_umma_kernel<128>, grid, dim3(THREADS), (size_t)Geo<128>::SMEM_BYTES, st, p);
-    else
-        launch_chained(prefill_attention_umma_kernel<64>, grid, dim3(THREADS), (size_t)Geo<64>::SMEM_BYTES, st, p);
+    launch_chained(prefill_attention_umma_kernel, grid, dim3(THREADS), (size_t)G::SMEM_BYTES, st, p);
 #ifdef GLMASR_EXPERIMENTS
     if (debug) {
         // timing experiment: where the soft-max warps of every CTA spent their cycles (averages over the CTAs)

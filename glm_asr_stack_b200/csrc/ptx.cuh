@@ -164,6 +164,15 @@ __device__ __forceinline__ void umma_bf16(uint32_t d_tmem, uint64_t adesc, uint6
         ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
         : "memory");
 }
+// Same with A in tensor memory: lane = row, bf16 pairs of consecutive k per 32-bit column (eight columns for K = 16).
+__device__ __forceinline__ void umma_bf16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+        ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
 // Block-scaled e2m1 x e2m1, one ue4m3 scale per 16 K-elements of each operand (NVFP4), K = 64.
 __device__ __forceinline__ void umma_nvfp4(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
                                            uint32_t accumulate, uint32_t sfa_tmem, uint32_t sfb_tmem) {
@@ -209,6 +218,13 @@ __device__ __forceinline__ void tmem_st_x32(uint32_t taddr, const uint32_t (&r)[
         "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
         "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};"
         ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
+        : "memory");
+}
+__device__ __forceinline__ void tmem_st_x16(uint32_t taddr, const uint32_t (&r)[16]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
+        "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
+        ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
         : "memory");
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
@@ -325,6 +341,18 @@ __device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t saddr) {
     d |= (uint64_t)2 << 61;                       // layout: SWIZZLE_128B
     return d;
 }
+// MN-major operand (the contiguous dimension is M or N): rows of 64 elements (128 bytes, 128B-swizzled) per k, as a TMA box
+// of 64 elements x k rows leaves them.  Eight k rows are 1024 bytes, the next 64 columns start box_bytes further on; a K
+// step of 16 is 2048 bytes.
+__device__ __forceinline__ uint64_t smem_desc_sw128_mn(uint32_t saddr, uint32_t box_bytes) {
+    uint64_t d = 0;
+    d |= (uint64_t)((saddr & 0x3FFFF) >> 4);
+    d |= (uint64_t)(box_bytes >> 4) << 16;        // leading byte offset: next 64 columns
+    d |= (uint64_t)(1024 >> 4) << 32;             // stride byte offset: next eight k rows
+    d |= (uint64_t)1 << 46;
+    d |= (uint64_t)2 << 61;
+    return d;
+}
 // Un-swizzled descriptor for a 32-row x 16-byte block stored row after row (16-byte pitch):
 // 8-row core matrices are 128 bytes apart.  Source of tcgen05.cp for one 128x4 scale chunk.
 __device__ __forceinline__ uint64_t smem_desc_sf_chunk(uint32_t saddr) {
@@ -343,6 +371,7 @@ __host__ __device__ constexpr uint32_t idesc_bf16(int m, int n) {
            | ((uint32_t)(n >> 3) << 17)   // N / 8
            | ((uint32_t)(m >> 4) << 24);  // M / 16
 }
+constexpr uint32_t kIdescBMnMajor = 1u << 16;   // B is MN-major (both operands are K-major without it)
 // Instruction descriptor, kind::mxf4nvf4: e2m1 x e2m1, ue4m3 scales, K = 64, K-major.
 __host__ __device__ constexpr uint32_t idesc_nvfp4(int m, int n) {
     return (1u << 7)                      // A format: e2m1

@@ -18,7 +18,7 @@ int *device_status_word();          // device pointer, 4 ints, zero-initialised;
 void *workspace(size_t bytes);      // grow-only private device workspace (slot 0)
 void *workspace_slot(int slot, size_t bytes);
 // Slots owned outside api.cu / decoder_step.cu (those two number their own, 0..31).
-enum : int { WS_ATTN_VT = 32, WS_ATTN_VT_COL = 33, WS_ATTN_DEBUG = 34 };
+enum : int { WS_ATTN_DEBUG = 34 };
 void free_all_private_state();
 void tail_forget_scales(const void *w_scales);   // decode_tail.cu: per-CTA re-tiled weight scales (nullptr: all)
 void encoder_forget_all();         // encoder.cu: per-store weight table, re-packed convolution weights, rotary table
