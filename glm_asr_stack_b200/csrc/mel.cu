@@ -8,11 +8,15 @@
 // The reference runs five launches and a cuFFT call per window, one window at a time.  Here a whole batch
 // of windows is two launches:
 //   mel_power_kernel      grid (frame tiles, windows): a CTA stages the tile's samples in shared memory,
-//                         applies the window, evaluates the DFT directly against a 400-entry twiddle table
-//                         (thread = frequency bin, 8 frames per pass in registers; N = 400 is not a power of
-//                         two and a tile's 32 x 201 outputs need only 5 M multiply-adds), then the power
-//                         spectrum times the filterbank in the reference's summation order, log10, the fp32
-//                         result to scratch and the tile's maximum to the window's maximum (atomic);
+//                         applies the window and evaluates the DFT directly against a 400-entry twiddle table, folded
+//                         twice: x[t] +- x[400 - t] (cosine and sine have that symmetry) leaves taps 0..200, and the
+//                         sums over even and odd taps give bin k as their sum and bin 200 - k as their difference, a
+//                         quarter of the multiply-adds and shorter sums.  A thread has two bins (and their mirror
+//                         images) of 8 frames.  Then the power spectrum times the filterbank in the reference's
+//                         summation order (16 frames per filter value read), log10, the fp32 result to scratch and the
+//                         tile's maximum to the window's maximum (atomic).  Bound: shared-memory reads and
+//                         multiply-adds of the DFT in balance, little else.  Unfolded, a bin a thread and 32 frames a
+//                         CTA it took 1750 us for sixteen 30 s windows and 196 us for one of 3.7 s, now 383 and 40;
 //   mel_normalize_kernel  clamp, affine map, bf16, written mel-major [128, n_frames] like the reference or
 //                         time-major [n_frames, 128] (what the encoder's convolution-as-GEMM reads).
 // The window maximum is the maximum over the WHOLE window.  The reference's second reduction pass
@@ -25,26 +29,31 @@
 #include <float.h>
 #include <stdint.h>
 
+#include <type_traits>
+
 #include "../../include/glmasr_fp4.h"
 #include "runtime.cuh"
 
 namespace glmasr {
 
 constexpr int kFft = 400, kHop = 160, kMels = 128, kBins = 201, kMaxFrames = 3000;
-constexpr int kTileFrames = 32;                                    // frames per CTA
-constexpr int kTileSamples = (kTileFrames - 1) * kHop + kFft;      // 5360
-constexpr int kMelThreads = 256;
+constexpr int kTileFrames = 16;                                    // frames per CTA
+constexpr int kTileSamples = (kTileFrames - 1) * kHop + kFft;      // 2800
+constexpr int kMelThreads = 128;
+constexpr int kSlots = 51;                                         // threads per 8 frames: bins i and i + 51 of 0..100
+constexpr int kRow = kTileFrames + 4;                              // floats per tap or bin: 16-byte rows, spread over the banks
 
 enum : int { WS_MEL_LOG = 35, WS_MEL_MAX = 36 };                   // private workspace slots of this file
 
 struct MelSmem {
-    float xw[kFft][kTileFrames];          // windowed frames, tap-major: 8 consecutive frames are two 16-byte loads
-    float2 tw[kFft];                      // (cos, sin)(2 pi j / 400)
+    float sum[kBins][kRow], dif[kBins][kRow];     // windowed x[t] + x[400 - t], x[t] - x[400 - t]
+    float power[kBins][kRow];                     // first the tile's raw samples (kTileSamples floats), then the power spectrum
+    float2 tw[kFft];                              // (cos, sin)(2 pi j / 400)
     float hann[kFft];
-    float power[kTileFrames][kBins + 3];  // first the tile's raw samples (kTileSamples floats), then the power spectrum
     float red[kMelThreads / 32];
 };
-static_assert(kTileSamples <= kTileFrames * (kBins + 3), "the raw samples of a tile are staged in the power array");
+static_assert(kTileSamples <= kBins * kRow, "the raw samples of a tile are staged in the power array");
+static_assert(kMelThreads == 64 * (kTileFrames / 8) && kMelThreads == kMels, "thread = (slot, 8 frames), then thread = mel bin");
 
 __device__ __forceinline__ void atomic_max_float(float *addr, float v) {
     // the cell starts as 0xFFFFFFFF: below every float in both orders used here
@@ -83,51 +92,100 @@ __global__ void __launch_bounds__(kMelThreads) mel_power_kernel(const float *__r
         raw[i] = (idx >= 0 && idx < ns) ? x[idx] : 0.0f;
     }
     __syncthreads();
-    for (int i = tid; i < kFft * kTileFrames; i += kMelThreads) {
-        const int t = i / kTileFrames, f = i - t * kTileFrames;
-        s.xw[t][f] = (f0 + f < n_frames) ? raw[f * kHop + t] * s.hann[t] : 0.0f;
-    }
-    __syncthreads();
-
-    // DFT: thread = bin k, eight frames per pass
-    if (tid < kBins) {
-        const int k = tid;
-#pragma unroll 1
-        for (int fg = 0; fg < kTileFrames; fg += 8) {
-            float re[8], im[8];
-#pragma unroll
-            for (int i = 0; i < 8; ++i) re[i] = im[i] = 0.0f;
-            int j = 0;                                   // (k * t) mod 400
-#pragma unroll 4
-            for (int t = 0; t < kFft; ++t) {
-                const float2 c = s.tw[j];
-                const float4 a = *reinterpret_cast<const float4 *>(&s.xw[t][fg]);
-                const float4 b = *reinterpret_cast<const float4 *>(&s.xw[t][fg + 4]);
-                // the sign of the imaginary part does not matter for the power
-#define GLMASR_MEL_ACC(i, xval) re[i] = fmaf(xval, c.x, re[i]), im[i] = fmaf(xval, c.y, im[i])
-                GLMASR_MEL_ACC(0, a.x); GLMASR_MEL_ACC(1, a.y); GLMASR_MEL_ACC(2, a.z); GLMASR_MEL_ACC(3, a.w);
-                GLMASR_MEL_ACC(4, b.x); GLMASR_MEL_ACC(5, b.y); GLMASR_MEL_ACC(6, b.z); GLMASR_MEL_ACC(7, b.w);
-#undef GLMASR_MEL_ACC
-                j += k;
-                if (j >= kFft) j -= kFft;
-            }
-#pragma unroll
-            for (int i = 0; i < 8; ++i) s.power[fg + i][k] = re[i] * re[i] + im[i] * im[i];
+    for (int f = 0; f < kTileFrames; ++f) {              // lanes over t: the frames overlap, 160 samples apart
+        const bool live = f0 + f < n_frames;
+        for (int t = tid; t < kBins; t += kMelThreads) {
+            const float a = live ? raw[f * kHop + t] * s.hann[t] : 0.0f;
+            const bool paired = t != 0 && t != kFft / 2;
+            const float b = live && paired ? raw[f * kHop + kFft - t] * s.hann[kFft - t] : 0.0f;
+            s.sum[t][f] = a + b;
+            s.dif[t][f] = paired ? a - b : 0.0f;         // the sine is zero at the unpaired taps
         }
     }
     __syncthreads();
 
-    // filterbank, log10, tile maximum: thread = mel bin m (two frame phases)
-    const int m = tid & (kMels - 1), phase = tid >> 7;
-    float tmax = -FLT_MAX;
-    for (int f = phase; f < kTileFrames && f0 + f < n_frames; f += kMelThreads / kMels) {
-        float p = 0.0f;
-#pragma unroll 4
-        for (int k = 0; k < kBins; ++k) p += s.power[f][k] * filters_t[k * kMels + m];      // mel.cu:141-149
-        const float v = log10f(p + 1e-10f);
-        logmel[((size_t)w * kMaxFrames + (size_t)(f0 + f)) * kMels + m] = v;
-        tmax = fmaxf(tmax, v);
+    const int slot = tid & 63, fg = (tid >> 6) * 8;
+    if (slot < kSlots) {
+        // [bin][even / odd taps][frame]
+        float re[2][2][8], im[2][2][8];
+#pragma unroll
+        for (int b = 0; b < 2; ++b)
+#pragma unroll
+            for (int i = 0; i < 8; ++i) re[b][0][i] = re[b][1][i] = im[b][0][i] = im[b][1][i] = 0.0f;
+        const int k0 = slot, k1 = slot + kSlots;         // k1 = 101 (a mirror image of 99) is computed and not stored
+        int j0 = 0, j1 = 0;                              // (k * t) mod 400
+        auto tap = [&](int t, auto odd) {
+            constexpr int o = decltype(odd)::value;
+            const float2 c0 = s.tw[j0], c1 = s.tw[j1];
+            const float4 sa = *reinterpret_cast<const float4 *>(&s.sum[t][fg]), sb = *reinterpret_cast<const float4 *>(&s.sum[t][fg + 4]);
+            const float4 da = *reinterpret_cast<const float4 *>(&s.dif[t][fg]), db = *reinterpret_cast<const float4 *>(&s.dif[t][fg + 4]);
+            const float sv[8] = {sa.x, sa.y, sa.z, sa.w, sb.x, sb.y, sb.z, sb.w};
+            const float dv[8] = {da.x, da.y, da.z, da.w, db.x, db.y, db.z, db.w};
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                re[0][o][i] = fmaf(sv[i], c0.x, re[0][o][i]);
+                im[0][o][i] = fmaf(dv[i], c0.y, im[0][o][i]);     // its sign does not matter for the power
+                re[1][o][i] = fmaf(sv[i], c1.x, re[1][o][i]);
+                im[1][o][i] = fmaf(dv[i], c1.y, im[1][o][i]);
+            }
+            j0 += k0;
+            if (j0 >= kFft) j0 -= kFft;
+            j1 += k1;
+            if (j1 >= kFft) j1 -= kFft;
+        };
+#pragma unroll 2
+        for (int t = 0; t < kFft / 2; t += 2) {
+            tap(t, std::integral_constant<int, 0>());
+            tap(t + 1, std::integral_constant<int, 1>());
+        }
+        tap(kFft / 2, std::integral_constant<int, 0>());
+#pragma unroll
+        for (int b = 0; b < 2; ++b) {
+            const int k = b == 0 ? k0 : k1;
+            if (k > kFft / 4) break;
+            float p[8], q[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const float r1 = re[b][0][i] + re[b][1][i], i1 = im[b][0][i] + im[b][1][i];
+                const float r2 = re[b][0][i] - re[b][1][i], i2 = im[b][0][i] - im[b][1][i];
+                p[i] = r1 * r1 + i1 * i1;
+                q[i] = r2 * r2 + i2 * i2;
+            }
+            *reinterpret_cast<float4 *>(&s.power[k][fg]) = make_float4(p[0], p[1], p[2], p[3]);
+            *reinterpret_cast<float4 *>(&s.power[k][fg + 4]) = make_float4(p[4], p[5], p[6], p[7]);
+            if (k != kFft / 4) {
+                *reinterpret_cast<float4 *>(&s.power[kFft / 2 - k][fg]) = make_float4(q[0], q[1], q[2], q[3]);
+                *reinterpret_cast<float4 *>(&s.power[kFft / 2 - k][fg + 4]) = make_float4(q[4], q[5], q[6], q[7]);
+            }
+        }
     }
+    __syncthreads();
+
+    // filterbank, log10, tile maximum: thread = mel bin, all frames of the tile
+    const int m = tid;
+    float p[kTileFrames];
+#pragma unroll
+    for (int f = 0; f < kTileFrames; ++f) p[f] = 0.0f;
+#pragma unroll 4
+    for (int k = 0; k < kBins; ++k) {                    // mel.cu:141-149
+        const float fw = filters_t[k * kMels + m];
+#pragma unroll
+        for (int f = 0; f < kTileFrames; f += 4) {
+            const float4 v = *reinterpret_cast<const float4 *>(&s.power[k][f]);
+            p[f] += v.x * fw;
+            p[f + 1] += v.y * fw;
+            p[f + 2] += v.z * fw;
+            p[f + 3] += v.w * fw;
+        }
+    }
+    float tmax = -FLT_MAX;
+#pragma unroll
+    for (int f = 0; f < kTileFrames; ++f)
+        if (f0 + f < n_frames) {
+            const float v = log10f(p[f] + 1e-10f);
+            logmel[((size_t)w * kMaxFrames + (size_t)(f0 + f)) * kMels + m] = v;
+            tmax = fmaxf(tmax, v);
+        }
     for (int off = 16; off > 0; off >>= 1) tmax = fmaxf(tmax, __shfl_xor_sync(0xFFFFFFFFu, tmax, off));
     if ((tid & 31) == 0) s.red[tid >> 5] = tmax;
     __syncthreads();
