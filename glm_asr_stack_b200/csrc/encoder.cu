@@ -42,68 +42,94 @@ enum : int { WS_E_NORM = 38, WS_E_QKV = 39, WS_E_FFN = 40, WS_E_POS = 41, WS_E_M
              WS_E_TMP = 45, WS_E_PROJ = 46, WS_E_ROPE = 47 };
 
 // --------------------------------------------------------------------------------------------
-// LayerNorm (reference: layernorm_kernel, Infer-engine/cuda/kernels.cu:299-345): one warp per row; lane i
-// adds x[i], x[i + 32], ... in that order, a shuffle-down tree, lane 0's total broadcast; the variance is a
-// second pass over (x - mean)^2; out = bf16(((x - mean) * inv_std) * w + b).  Eight rows per CTA.  out may
-// alias x (a warp has its whole row in shared memory before it writes any of it).
+// LayerNorm (reference: layernorm_kernel, Infer-engine/cuda/kernels.cu:299-345): lane i of a warp adds x[i], x[i + 32],
+// ... in that order, a shuffle-down tree, lane 0's total broadcast; the variance is a second pass over (x - mean)^2;
+// out = bf16(((x - mean) * inv_std) * w + b).  out may alias x (a warp has its rows in shared memory before it writes).
+// A warp takes two rows: its sixteen lanes per row each carry two neighbouring lanes of that order, so both sums read
+// shared memory in 32-bit words; the last step is element-wise and works on 16-byte pieces.  Same bits as one row per
+// warp with three passes of 2-byte shared loads, which was bound by the shared-memory pipe (24000 x 1280 in the encoder:
+// 50 us a launch, now 35; a copy of the same bytes takes 27).  Words kept in registers between the sums cost half the
+// resident warps: 40 us.
 // --------------------------------------------------------------------------------------------
-template <int MAXE>
-__global__ void __launch_bounds__(256) layernorm_kernel(__nv_bfloat16 *out, const __nv_bfloat16 *x, const __nv_bfloat16 *weight,
-                                                        const __nv_bfloat16 *bias, float eps, int rows, int dim) {
-    // Rows move between global and shared memory in 16-byte pieces (dim % 8 == 0, 16-byte aligned rows); the
-    // arithmetic reads the warp's row from shared memory in the reference's lane-strided order.  weight and bias
-    // are staged once per CTA.
+static constexpr int kLnWarps = 4, kLnRows = 2 * kLnWarps;
+static size_t ln_smem_bytes(int dim) { return (size_t)dim * 4 + (size_t)kLnRows * (dim * 2 + 64); }
+
+__global__ void __launch_bounds__(kLnWarps * 32, 8) layernorm_kernel(__nv_bfloat16 *out, const __nv_bfloat16 *x,
+                                                                  const __nv_bfloat16 *weight, const __nv_bfloat16 *bias,
+                                                                  float eps, int rows, int dim) {
     extern __shared__ __align__(16) uint8_t ln_smem[];
-    __nv_bfloat16 *w_s = reinterpret_cast<__nv_bfloat16 *>(ln_smem);
-    __nv_bfloat16 *b_s = w_s + dim;
+    uint4 *w_s = reinterpret_cast<uint4 *>(ln_smem), *b_s = w_s + (dim >> 3);
     pdl_launch_dependents();
-    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, row = blockIdx.x * 8 + wib;
-    __nv_bfloat16 *row_s = b_s + dim + (size_t)wib * dim;
-    const int vecs = dim >> 3;
-    for (int i = threadIdx.x; i < vecs; i += 256) {
-        reinterpret_cast<uint4 *>(w_s)[i] = reinterpret_cast<const uint4 *>(weight)[i];
-        reinterpret_cast<uint4 *>(b_s)[i] = bias != nullptr ? reinterpret_cast<const uint4 *>(bias)[i] : make_uint4(0u, 0u, 0u, 0u);
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, vecs = dim >> 3;
+    const int row0 = blockIdx.x * kLnRows + wib * 2;
+    uint8_t *rows_s = ln_smem + (size_t)dim * 4 + (size_t)wib * 2 * (dim * 2 + 64);     // 64 bytes apart: other banks
+    for (int i = threadIdx.x; i < vecs; i += kLnWarps * 32) {
+        w_s[i] = reinterpret_cast<const uint4 *>(weight)[i];
+        b_s[i] = bias != nullptr ? reinterpret_cast<const uint4 *>(bias)[i] : make_uint4(0u, 0u, 0u, 0u);
     }
     pdl_wait();
-    if (row < rows) {
-        const uint4 *xr = reinterpret_cast<const uint4 *>(x + (size_t)row * dim);
-        for (int i = lane; i < vecs; i += 32) reinterpret_cast<uint4 *>(row_s)[i] = xr[i];
-    }
+#pragma unroll
+    for (int r = 0; r < 2; ++r)
+        if (row0 + r < rows) {
+            const uint4 *xr = reinterpret_cast<const uint4 *>(x + (size_t)(row0 + r) * dim);
+            for (int i = lane; i < vecs; i += 32) reinterpret_cast<uint4 *>(rows_s + r * (dim * 2 + 64))[i] = xr[i];
+        }
     __syncthreads();
-    if (row >= rows) return;
-    // three passes over the row in shared memory (kept out of registers: eight CTAs per SM stay resident)
-    float sum = 0.0f;
+    if (row0 >= rows) return;
+    const int l = lane & 15;
+    const uint32_t *words = reinterpret_cast<const uint32_t *>(rows_s + (lane >> 4) * (dim * 2 + 64));
+    const int n_words = dim / 2 > l ? (dim / 2 - l + 15) / 16 : 0;
+    float s0 = 0.0f, s1 = 0.0f;
 #pragma unroll 8
-    for (int j = 0; j < MAXE; ++j) {
-        const int i = lane + 32 * j;
-        if (i < dim) sum += __bfloat162float(row_s[i]);
+    for (int n = 0; n < n_words; ++n) {
+        const uint32_t v = words[16 * n + l];
+        s0 += __uint_as_float(v << 16);
+        s1 += __uint_as_float(v & 0xFFFF0000u);
     }
-    for (int off = 16; off > 0; off >>= 1) sum += __shfl_down_sync(0xFFFFFFFFu, sum, off);
-    sum = __shfl_sync(0xFFFFFFFFu, sum, 0);
-    const float mean = sum / dim;
-    float sum_sq = 0.0f;
+    auto tree = [&](float a, float b) {
+#pragma unroll
+        for (int off = 8; off > 0; off >>= 1) {
+            a += __shfl_down_sync(0xFFFFFFFFu, a, off, 16);
+            b += __shfl_down_sync(0xFFFFFFFFu, b, off, 16);
+        }
+        return a + b;
+    };
+    const float mean = __shfl_sync(0xFFFFFFFFu, tree(s0, s1), 0, 16) / dim;
+    s0 = s1 = 0.0f;
 #pragma unroll 8
-    for (int j = 0; j < MAXE; ++j) {
-        const int i = lane + 32 * j;
-        if (i < dim) {
-            const float d = __bfloat162float(row_s[i]) - mean;
-            sum_sq += d * d;
+    for (int n = 0; n < n_words; ++n) {
+        const uint32_t v = words[16 * n + l];
+        const float d0 = __uint_as_float(v << 16) - mean, d1 = __uint_as_float(v & 0xFFFF0000u) - mean;
+        s0 += d0 * d0;
+        s1 += d1 * d1;
+    }
+    const float inv = 1.0f / sqrtf(__shfl_sync(0xFFFFFFFFu, tree(s0, s1), 0, 16) / dim + eps);
+    float m[2], is[2];
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+        m[r] = __shfl_sync(0xFFFFFFFFu, mean, 16 * r);
+        is[r] = __shfl_sync(0xFFFFFFFFu, inv, 16 * r);
+    }
+    for (int i = lane; i < vecs; i += 32) {
+        const uint4 w4 = w_s[i], b4 = b_s[i];
+        const uint32_t w[4] = {w4.x, w4.y, w4.z, w4.w}, b[4] = {b4.x, b4.y, b4.z, b4.w};
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            if (row0 + r >= rows) break;
+            const uint4 x4 = reinterpret_cast<const uint4 *>(rows_s + r * (dim * 2 + 64))[i];
+            const uint32_t xs[4] = {x4.x, x4.y, x4.z, x4.w};
+            uint32_t o[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const float lo = (__uint_as_float(xs[e] << 16) - m[r]) * is[r];
+                const float hi = (__uint_as_float(xs[e] & 0xFFFF0000u) - m[r]) * is[r];
+                const __nv_bfloat162 p = __floats2bfloat162_rn(lo * __uint_as_float(w[e] << 16) + __uint_as_float(b[e] << 16),
+                                                               hi * __uint_as_float(w[e] & 0xFFFF0000u) + __uint_as_float(b[e] & 0xFFFF0000u));
+                o[e] = *reinterpret_cast<const uint32_t *>(&p);
+            }
+            reinterpret_cast<uint4 *>(out + (size_t)(row0 + r) * dim)[i] = make_uint4(o[0], o[1], o[2], o[3]);
         }
     }
-    for (int off = 16; off > 0; off >>= 1) sum_sq += __shfl_down_sync(0xFFFFFFFFu, sum_sq, off);
-    sum_sq = __shfl_sync(0xFFFFFFFFu, sum_sq, 0);
-    const float inv_std = 1.0f / sqrtf(sum_sq / dim + eps);
-#pragma unroll 8
-    for (int j = 0; j < MAXE; ++j) {
-        const int i = lane + 32 * j;
-        if (i < dim) {
-            const float val = (__bfloat162float(row_s[i]) - mean) * inv_std;
-            row_s[i] = __float2bfloat16(val * __bfloat162float(w_s[i]) + __bfloat162float(b_s[i]));
-        }
-    }
-    __syncwarp();
-    uint4 *orow = reinterpret_cast<uint4 *>(out + (size_t)row * dim);
-    for (int i = lane; i < vecs; i += 32) orow[i] = reinterpret_cast<const uint4 *>(row_s)[i];
 }
 
 // any width (three passes over global memory), same arithmetic; in place is fine here too: a lane reads and writes
@@ -140,12 +166,12 @@ __global__ void layernorm_generic_kernel(__nv_bfloat16 *out, const __nv_bfloat16
 void launch_layernorm(__nv_bfloat16 *out, const __nv_bfloat16 *x, const __nv_bfloat16 *weight, const __nv_bfloat16 *bias,
                       float eps, int rows, int dim, cudaStream_t st) {
     if (rows <= 0) return;
-    const dim3 grid((rows + 7) / 8);
     const bool vec = (dim % 8) == 0 && (((uintptr_t)out | (uintptr_t)x | (uintptr_t)weight | (uintptr_t)bias) & 15) == 0;
-    if (dim <= 32 * 40 && vec)       // the row fits the registers of a warp (the encoder's 1280)
-        launch_chained(layernorm_kernel<40>, grid, dim3(256), (size_t)dim * 2 * 10, st, out, x, weight, bias, eps, rows, dim);
+    if (dim <= 1280 && vec)          // eight rows fit 48 KB of shared memory (the encoder's 1280)
+        launch_chained(layernorm_kernel, dim3((rows + kLnRows - 1) / kLnRows), dim3(kLnWarps * 32), ln_smem_bytes(dim), st, out, x,
+                       weight, bias, eps, rows, dim);
     else
-        launch_chained(layernorm_generic_kernel, grid, dim3(256), (size_t)0, st, out, x, weight, bias, eps, rows, dim);
+        launch_chained(layernorm_generic_kernel, dim3((rows + 7) / 8), dim3(256), (size_t)0, st, out, x, weight, bias, eps, rows, dim);
     note_launches(1);
 }
 

@@ -56,6 +56,17 @@ def test_layernorm(ops, ref, rows, dim):
         assert np.array_equal(got, bits_of(ref.layernorm(to_dev_bf16(x), to_dev_bf16(w), to_dev_bf16(b))))
 
 
+@pytest.mark.parametrize("rows,dim", [(1, 8), (7, 40), (8, 1272), (9, 1280), (18, 96)])
+def test_layernorm_two_rows_per_warp_same_bits(ops, rows, dim):
+    """The vectorised kernel (two rows per warp) adds in the order of the kernel that takes any alignment: equal bits, at
+    odd rows and at widths that end inside a warp's words."""
+    rng = np.random.default_rng(dim)
+    x, w, b = to_dev_bf16(rb(rng, (rows, dim), 2.0, 0.3)), to_dev_bf16(rb(rng, (dim,), 0.1, 1.0)), to_dev_bf16(rb(rng, (dim,), 0.1))
+    odd = torch.empty(rows * dim + 1, dtype=x.dtype, device="cuda")[1:].view(rows, dim)       # two bytes off: the other kernel
+    odd.copy_(x)
+    assert torch.equal(ops.layernorm(x, w, b).view(torch.int16), ops.layernorm(odd, w, b).view(torch.int16))
+
+
 def test_gelu_and_residual_add_bias(ops, ref):
     rng = np.random.default_rng(3)
     x = rb(rng, (333, 77), 2.0)
