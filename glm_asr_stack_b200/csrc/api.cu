@@ -77,7 +77,14 @@ int *device_status_word() {
 // 0: never, 1: everywhere except the chunked host-buffer call, 2: everywhere
 static int g_pdl_mode = -1;
 static bool g_pdl_suppressed = false;      // set while the chunked host-buffer call enqueues its kernels
+static bool g_plain = false, g_settled = false;
+PlainLaunch::PlainLaunch(bool on) : before(g_plain) { g_plain = g_plain || on; }
+PlainLaunch::~PlainLaunch() { g_plain = before; }
+SettledWeights::SettledWeights(bool on) : before(g_settled) { g_settled = g_settled || on; }
+SettledWeights::~SettledWeights() { g_settled = before; }
+bool weights_settled() { return g_settled; }
 bool pdl_enabled() {
+    if (g_plain) return false;
     if (g_pdl_mode < 0) {
         const char *e = getenv("GLMASR_PDL");
         g_pdl_mode = (e && e[0] >= '0' && e[0] <= '2') ? e[0] - '0' : 1;
@@ -530,8 +537,8 @@ static int run_simt(const FusedArgs &a) {
 static int g_route_rows = 0;
 
 // The resident bf16 copy of one FP4 weight [N, K]; nullptr when it cannot be kept (no scale tensor to key it by,
-// budget spent, allocation refused).
-static const __nv_bfloat16 *resident_bf16_weight(const glmasr_fp4_weight &w, int K) {
+// budget spent, allocation refused).  *made is set when this call launched the kernel that writes it.
+static const __nv_bfloat16 *resident_bf16_weight(const glmasr_fp4_weight &w, int K, bool *made) {
     if (w.w_scales == nullptr || w.w_packed == nullptr || w.N <= 0 || K <= 0) return nullptr;
     auto it = g_resident.find(w.w_scales);
     if (it != g_resident.end()) {
@@ -551,6 +558,7 @@ static const __nv_bfloat16 *resident_bf16_weight(const glmasr_fp4_weight &w, int
     ++g_launches;
     g_resident[w.w_scales] = r;
     g_resident_bytes += bytes;
+    *made = true;
     return r.w;
 }
 
@@ -589,6 +597,7 @@ static int run_skinny(const FusedArgs &a, const __nv_bfloat16 *norm_w = nullptr,
     p.residual = a.residual;
     p.bias = a.bias;
     p.ldo = a.ldo;
+    p.early_weights = a.mode == GEMM_W4A4 || weights_settled() ? 1 : 0;
     p.status = device_status_word();
     profile_bracket_begin(2.0 * a.M * n_rows * a.K, 0.5625 * n_rows * a.K + 2.0 * a.M * (a.K + total_out_cols(a)));
     if (launch_skinny_linear(p, num_sms(), g_stream) != cudaSuccess) return -1;
@@ -695,9 +704,9 @@ static int run_fused(const FusedArgs &a) {
     // small dependent stages (gate|up at 256 rows: 43 us against ~12)
     if (a.mode == GEMM_W4A16 && resident_budget_bytes() > 0) {
         const __nv_bfloat16 *wb[kMaxSegments];
-        bool all = true;
+        bool all = true, made = false;
         for (int i = 0; i < a.num_w && all; ++i) {
-            wb[i] = resident_bf16_weight(a.w[i], a.K);
+            wb[i] = resident_bf16_weight(a.w[i], a.K, &made);
             all = wb[i] != nullptr;
         }
         if (all) {
@@ -708,7 +717,8 @@ static int run_fused(const FusedArgs &a) {
                 b.n_bf16[i] = a.w[i].N;
             }
             b.w = nullptr;
-            b.const_weights = true;         // the copy is made by an ordinary launch, which ends before anything behind it starts
+            b.const_weights = true;
+            PlainLaunch plain(made);        // later calls fetch the copy early
             return run_fused(b);
         }
     }

@@ -825,25 +825,29 @@ extern "C" void decoder_decode_step_batched(void *handle, const void *ws_v, uint
 
     // the rotary angles depend on the positions only: one evaluation for all layers
     float *rope_angles = (float *)workspace_slot(WS_D_ANGLES, (size_t)M * HD * sizeof(float));
-    if (launch_step_setup((__nv_bfloat16 *)hid, query_ptrs, M, H, h_slot.data(), d_slot, h_total.data(), d_total, h_rows.data(),
-                          pool->d_block_tables, d_bt, pool->max_blocks_per_seq, d_seq_lens, rope_angles, HD, st)) {
-        note_launches(1);
-        if (!contiguous) GLMASR_CUDA_CHECK(cudaMemcpyAsync(d_ptrs, query_ptrs, (size_t)M * sizeof(void *), cudaMemcpyHostToDevice, st));
-    } else {
-        GLMASR_CUDA_CHECK(cudaMemcpyAsync(d_slot, h_slot.data(), (size_t)M * sizeof(int64_t), cudaMemcpyHostToDevice, st));
-        GLMASR_CUDA_CHECK(cudaMemcpyAsync(d_total, h_total.data(), (size_t)M * sizeof(int), cudaMemcpyHostToDevice, st));
-        GLMASR_CUDA_CHECK(cudaMemcpyAsync(d_rows, h_rows.data(), (size_t)M * sizeof(int), cudaMemcpyHostToDevice, st));
-        if (contiguous) {
-            GLMASR_CUDA_CHECK(cudaMemcpyAsync(hid, query_ptrs[0], (size_t)M * H * 2, cudaMemcpyDeviceToDevice, st));
+    {
+        PlainLaunch plain(true);        // the kernels behind it fetch weights and cached rows early
+        if (launch_step_setup((__nv_bfloat16 *)hid, query_ptrs, M, H, h_slot.data(), d_slot, h_total.data(), d_total, h_rows.data(),
+                              pool->d_block_tables, d_bt, pool->max_blocks_per_seq, d_seq_lens, rope_angles, HD, st)) {
+            note_launches(1);
+            if (!contiguous) GLMASR_CUDA_CHECK(cudaMemcpyAsync(d_ptrs, query_ptrs, (size_t)M * sizeof(void *), cudaMemcpyHostToDevice, st));
         } else {
-            GLMASR_CUDA_CHECK(cudaMemcpyAsync(d_ptrs, query_ptrs, (size_t)M * sizeof(void *), cudaMemcpyHostToDevice, st));
-            launch_gather_rows((__nv_bfloat16 *)hid, (const __nv_bfloat16 *const *)d_ptrs, M, H, st);
+            GLMASR_CUDA_CHECK(cudaMemcpyAsync(d_slot, h_slot.data(), (size_t)M * sizeof(int64_t), cudaMemcpyHostToDevice, st));
+            GLMASR_CUDA_CHECK(cudaMemcpyAsync(d_total, h_total.data(), (size_t)M * sizeof(int), cudaMemcpyHostToDevice, st));
+            GLMASR_CUDA_CHECK(cudaMemcpyAsync(d_rows, h_rows.data(), (size_t)M * sizeof(int), cudaMemcpyHostToDevice, st));
+            if (contiguous) {
+                GLMASR_CUDA_CHECK(cudaMemcpyAsync(hid, query_ptrs[0], (size_t)M * H * 2, cudaMemcpyDeviceToDevice, st));
+            } else {
+                GLMASR_CUDA_CHECK(cudaMemcpyAsync(d_ptrs, query_ptrs, (size_t)M * sizeof(void *), cudaMemcpyHostToDevice, st));
+                launch_gather_rows((__nv_bfloat16 *)hid, (const __nv_bfloat16 *const *)d_ptrs, M, H, st);
+            }
+            launch_gather_block_tables(d_bt, pool->d_block_tables, d_rows, M, pool->max_blocks_per_seq, st);
+            // the vectors above are pageable host memory: the async copies have completed staging on return
+            if (launch_rope_angles(rope_angles, d_seq_lens, M, HD, st)) note_launches(1);
+            else rope_angles = nullptr;
         }
-        launch_gather_block_tables(d_bt, pool->d_block_tables, d_rows, M, pool->max_blocks_per_seq, st);
-        // the vectors above are pageable host memory: the async copies have completed staging on return
-        if (launch_rope_angles(rope_angles, d_seq_lens, M, HD, st)) note_launches(1);
-        else rope_angles = nullptr;
     }
+    SettledWeights settled(true);
 
     // the layer tail (o .. next layer's q|k|v) as one co-resident launch where it applies
     const bool tail = tail_enabled() && M <= 256;
@@ -1019,8 +1023,12 @@ extern "C" void decoder_prefill_paged_batched(void *handle, const void *ws_v, ui
     GLMASR_CUDA_CHECK(cudaMemcpyAsync(d_pos, h_pos.data(), (size_t)M * sizeof(int), cudaMemcpyHostToDevice, st));
     GLMASR_CUDA_CHECK(cudaMemcpyAsync(d_meta, h_meta.data(), (size_t)2 * num_seqs * sizeof(int), cudaMemcpyHostToDevice, st));
     float *rope_angles = (float *)workspace_slot(WS_D_ANGLES, (size_t)M * HD * sizeof(float));
-    if (launch_rope_angles(rope_angles, d_pos, M, HD, st)) note_launches(1);
-    else rope_angles = nullptr;
+    {
+        PlainLaunch plain(true);
+        if (launch_rope_angles(rope_angles, d_pos, M, HD, st)) note_launches(1);
+        else rope_angles = nullptr;
+    }
+    SettledWeights settled(rope_angles != nullptr);
 
     uint16_t *hid = hidden;
     for (int l = 0; l < L; ++l) {

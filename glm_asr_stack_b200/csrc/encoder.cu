@@ -544,7 +544,10 @@ static void encoder_layers(const glmasr_WeightStore *ws, const glmasr_ModelConfi
     uint16_t *qkv = (uint16_t *)workspace_slot(WS_E_QKV, (size_t)M * 3 * H * 2);
     uint16_t *ffn = (uint16_t *)workspace_slot(WS_E_FFN, (size_t)M * F * 2);
     int *row_pos = (int *)workspace_slot(WS_E_POS, (size_t)M * sizeof(int));
-    launch_chained(fill_row_positions_kernel, dim3(8, num_seqs), dim3(256), (size_t)0, st, row_pos, d_offsets, d_lens, num_seqs);
+    {
+        PlainLaunch plain(true);        // the GEMMs behind it fetch their weights early
+        launch_chained(fill_row_positions_kernel, dim3(8, num_seqs), dim3(256), (size_t)0, st, row_pos, d_offsets, d_lens, num_seqs);
+    }
     note_launches(1);
     for (int l = 0; l < L; ++l) {
         const EncLayerRef &W = R.layers[l];
@@ -633,10 +636,13 @@ extern "C" void conv1d_forward(uint16_t *out, const uint16_t *input, const uint1
     uint16_t *col = (uint16_t *)workspace_slot(WS_E_COL, (size_t)out_len * K * 2);
     uint16_t *tmp = (uint16_t *)workspace_slot(WS_E_TMP, (size_t)out_len * out_ch * 2);
     const long long total = (long long)out_len * K;
-    launch_chained(im2col_channel_major_kernel, dim3((unsigned)((total + 255) / 256)), dim3(256), (size_t)0, st,
-                   (__nv_bfloat16 *)col, (const __nv_bfloat16 *)input, in_ch, seq_len, out_len, kernel_size, stride, padding);
-    note_launches(1);
     const uint16_t *w2 = packed_conv_weight(weight, out_ch, in_ch, kernel_size, st);
+    {
+        PlainLaunch plain(true);        // the GEMM behind it fetches the weight early
+        launch_chained(im2col_channel_major_kernel, dim3((unsigned)((total + 255) / 256)), dim3(256), (size_t)0, st,
+                       (__nv_bfloat16 *)col, (const __nv_bfloat16 *)input, in_ch, seq_len, out_len, kernel_size, stride, padding);
+    }
+    note_launches(1);
     GLMASR_CHECK(gemm(tmp, out_ch, col, K, w2, out_ch, nullptr, EPI_STORE, nullptr, out_len, K) == 0,
                  "conv1d_forward: unsupported shape (in_ch %d, out_ch %d, kernel %d)", in_ch, out_ch, kernel_size);
     if (bias != nullptr) {
@@ -751,8 +757,11 @@ extern "C" int glmasr_audio_encode_batched(const void *ws_v, const void *cfg_v, 
     const int K1 = 3 * MELS, K2 = 3 * H;
     uint16_t *col = (uint16_t *)workspace_slot(WS_E_COL, (size_t)W * (size_t)((size_t)t1_max * K1 > (size_t)t2_max * K2 ? (size_t)t1_max * K1 : (size_t)t2_max * K2) * 2);
     uint16_t *c1 = (uint16_t *)workspace_slot(WS_E_CONV1, (size_t)W * t1_max * H * 2);
-    launch_chained(im2col_time_major_kernel, dim3(1, t1_max, W), dim3(64), (size_t)0, st, (__nv_bfloat16 *)col,
-                   (const __nv_bfloat16 *)mel, MELS, mel_stride, d_len1, t1_max, 3, 1, 1);
+    {
+        PlainLaunch plain(true);        // the GEMMs behind it fetch their weights early
+        launch_chained(im2col_time_major_kernel, dim3(1, t1_max, W), dim3(64), (size_t)0, st, (__nv_bfloat16 *)col,
+                       (const __nv_bfloat16 *)mel, MELS, mel_stride, d_len1, t1_max, 3, 1, 1);
+    }
     note_launches(1);
     if (gemm(c1, H, col, K1, c1p, H, c1b, EPI_GELU, nullptr, W * t1_max, K1) != 0) return -1;
     // conv2 + GELU: [W * t2_max, 3 H] x [H, 3 H]^T -> the encoder's hidden state [W][rows_enc][H]

@@ -174,8 +174,9 @@ __global__ void __launch_bounds__(kThreadsSk, 2) skinny_linear_kernel(const __gr
                 bulk_load_1d(dst + 16 * w_pitch + rr * s_pitch, p.ws[seg] + (size_t)(row + rr) * (p.K / 16), p.K / 16, bar);
         }
     };
+    if (!p.early_weights) pdl_wait();
     for (int r = 0; r < p.groups && r < rounds; ++r) issue_round(r);
-    pdl_wait();
+    if (p.early_weights) pdl_wait();
 
     const int chunks = p.K >> 7;
     float ss[NT];

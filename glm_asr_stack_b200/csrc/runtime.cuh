@@ -59,6 +59,23 @@ void profile_bracket_end();
 // dependencies are exactly those of an ordinary stream.  GLMASR_PDL=0 turns the attribute off.
 bool pdl_enabled();
 
+// A kernel that fetches weights ahead of pdl_wait() needs more than stream order: whatever wrote them has to have
+// completed before the kernel in FRONT of it started.  An ordinary launch (no attribute) starts when everything before
+// it has completed, so one such launch between the writer and the chain settles that for all kernels behind it.
+// PlainLaunch makes the launches of its scope ordinary ones; SettledWeights marks the scope of a driver whose first
+// launch was ordinary, in which the caller's packed weights may be fetched early.
+struct PlainLaunch {
+    explicit PlainLaunch(bool on);
+    ~PlainLaunch();
+    bool before;
+};
+struct SettledWeights {
+    explicit SettledWeights(bool on);
+    ~SettledWeights();
+    bool before;
+};
+bool weights_settled();
+
 #ifdef __CUDACC__
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
