@@ -654,10 +654,12 @@ static int run_cluster(const FusedArgs &a) {
         if (i == 0 || !silu) tiles += p.seg_tiles[i];
         n_rows += a.n_bf16[i];
     }
-    // the single-CTA kernel: about 0.25 us per 64-wide k block of a 128 x 128 tile, one tile per SM and round
+    // the single-CTA kernel, in a chain of launches: 5.5 us and 0.2 us per 64-wide k block of a 128 x 128 tile, one tile per
+    // SM and round; gate and up are one tile of twice that (measured: 185 x 1280 x 1280 11 us, 185 x 3840 x 1280 9.4,
+    // 173 x 2048 x 6144 24.7, gate|up of 19 and of 173 rows with K = 2048 19.5; this kernel: 8.9, -, 17.8, 12.8 for 19 rows)
     const double cluster_ns = choose_cluster_gemm(p, tiles);
-    const double rounds = ((a.M + 127) / 128 * (silu ? 2 * ((a.n_bf16[0] + 127) / 128) : tiles) + num_sms() - 1) / num_sms();
-    if (cluster_ns == 0.0 || cluster_ns > 3000.0 + 250.0 * p.k_blocks * rounds) return 1;
+    const int rounds = ((a.M + 127) / 128 * (silu ? (a.n_bf16[0] + 127) / 128 : tiles) + num_sms() - 1) / num_sms();
+    if (cluster_ns == 0.0 || cluster_ns > 5500.0 + (silu ? 400.0 : 200.0) * p.k_blocks * rounds) return 1;
     for (int i = 0; i < a.num_w; ++i)
         if (!make_tmap(&p.tm_w[i], a.w_bf16[i], CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)a.K, (uint64_t)a.n_bf16[i],
                        (uint64_t)a.K * 2, 64, silu ? 64 : 128, true))
