@@ -77,12 +77,18 @@ int *device_status_word() {
 // 0: never, 1: everywhere except the chunked host-buffer call, 2: everywhere
 static int g_pdl_mode = -1;
 static bool g_pdl_suppressed = false;      // set while the chunked host-buffer call enqueues its kernels
-static bool g_plain = false, g_settled = false;
+static thread_local bool g_plain = false, g_settled = false;
 PlainLaunch::PlainLaunch(bool on) : before(g_plain) { g_plain = g_plain || on; }
 PlainLaunch::~PlainLaunch() { g_plain = before; }
 SettledWeights::SettledWeights(bool on) : before(g_settled) { g_settled = g_settled || on; }
 SettledWeights::~SettledWeights() { g_settled = before; }
 bool weights_settled() { return g_settled; }
+static thread_local bool g_late_asked = false, g_late_taken = false;
+LateTrigger::LateTrigger() { g_late_asked = true; g_late_taken = false; }
+LateTrigger::~LateTrigger() { g_late_asked = false; }
+bool late_trigger_asked() { return g_late_asked; }
+void note_late_trigger(bool taken) { g_late_taken = taken; }
+bool late_trigger_taken() { return g_late_taken; }
 bool pdl_enabled() {
     if (g_plain) return false;
     if (g_pdl_mode < 0) {
@@ -600,7 +606,9 @@ static int run_skinny(const FusedArgs &a, const __nv_bfloat16 *norm_w = nullptr,
     p.early_weights = a.mode == GEMM_W4A4 || weights_settled() ? 1 : 0;
     p.status = device_status_word();
     profile_bracket_begin(2.0 * a.M * n_rows * a.K, 0.5625 * n_rows * a.K + 2.0 * a.M * (a.K + total_out_cols(a)));
+    p.late_trigger = late_trigger_asked() ? 1 : 0;
     if (launch_skinny_linear(p, num_sms(), g_stream) != cudaSuccess) return -1;
+    note_late_trigger(p.late_trigger != 0);
     profile_bracket_end();
     ++g_launches;
     return 0;
@@ -675,13 +683,16 @@ static int run_cluster(const FusedArgs &a) {
     p.status = device_status_word();
     profile_bracket_begin(2.0 * a.M * n_rows * a.K, 2.0 * n_rows * a.K + 2.0 * a.M * (a.K + total_out_cols(a)) +
                                                         (a.epi == EPI_RESIDUAL ? 2.0 * a.M * total_out_cols(a) : 0.0));
+    p.late_trigger = late_trigger_asked() ? 1 : 0;
     if (launch_cluster_gemm(p, g_stream) != cudaSuccess) return -1;
+    note_late_trigger(p.late_trigger != 0);
     profile_bracket_end();
     ++g_launches;
     return 0;
 }
 
 static int run_fused(const FusedArgs &a) {
+    note_late_trigger(false);
     if (a.M <= 0 || a.K <= 0) return -1;
     if (a.mode != GEMM_BF16) {
         if (a.num_w < 1 || a.num_w > kMaxSegments) return -1;

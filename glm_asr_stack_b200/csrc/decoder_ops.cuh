@@ -46,14 +46,16 @@ bool launch_paged_decode_attention_mma(__nv_bfloat16 *out, int ldo, const __nv_b
                                        int num_kv_heads, int head_dim, int block_size, int max_blocks_per_seq,
                                        cudaStream_t st, uint8_t *q_packed = nullptr, uint8_t *q_sf = nullptr,
                                        float q_input_scale = 0.0f);
-// RoPE + cache write + attention of a small decode batch as one launch, context cut over clusters; angles as
-// launch_rope_angles writes them, max_len = the longest context (tokens attended).  False when another route is better or
-// the layout is not covered (nothing launched).
+// RoPE + cache write + attention of a decode batch as one launch, the context of a small batch cut over clusters; angles as
+// launch_rope_angles writes them, max_len = the longest context (tokens attended).  early_cache: everything but the q|k|v
+// projection in front has completed when this kernel starts (LateTrigger).  With q_packed the result is written as the
+// quantised operand of the o projection instead of bf16.  False when the layout is not covered (nothing launched).
 bool launch_paged_decode_split(__nv_bfloat16 *out, int ldo, const __nv_bfloat16 *qkv, int ld, int k_col, int v_col,
                                const float *angles, const int64_t *slot_mapping, __nv_bfloat16 *key_cache,
                                __nv_bfloat16 *value_cache, const int *block_tables, const int *seq_lens, int num_seqs,
                                int num_q_heads, int num_kv_heads, int head_dim, int block_size, int max_blocks_per_seq,
-                               int max_len, cudaStream_t st);
+                               int max_len, cudaStream_t st, bool early_cache, uint8_t *q_packed = nullptr, uint8_t *q_sf = nullptr,
+                               float q_input_scale = 0.0f);
 // Everything a decode step needs on the device before its first layer, in one launch: hidden rows gathered from rows[i]
 // (16-byte aligned, dim % 8 == 0), cache slots, lengths, block-table rows and rotary angles of the cached positions.
 // The host values travel as kernel parameters.  False when the batch is too large for that.

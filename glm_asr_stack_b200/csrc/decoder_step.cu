@@ -867,35 +867,44 @@ extern "C" void decoder_decode_step_batched(void *handle, const void *ws_v, uint
         __nv_bfloat16 *v_base = (__nv_bfloat16 *)pool->v_cache + (size_t)l * pool->layer_stride;
 
         // q | k | v into one [M, H + 2 KV] buffer
-        int glue = have_qkv ? 0 : project_qkv(R, hid, B, M, H, KV, st);
+        int glue = 0;
+        bool early_cache = false;       // attention may read the cache and the step's tables ahead of its dependency wait
+        if (!have_qkv) {
+            LateTrigger late;
+            glue = project_qkv(R, hid, B, M, H, KV, st);
+            early_cache = late_trigger_taken();
+        }
         have_qkv = false;
         // attention writes the o projection's quantised operand itself when that projection runs in W4A4
         const bool o_q = takes_quantised_input(R.o) && R.o.K == H && !attn_scalar_forced();
-        // a small batch whose o projection takes bf16: RoPE, cache write and attention in one launch
-        if (!o_q && !attn_scalar_forced() &&
-            launch_paged_decode_split((__nv_bfloat16 *)att, H, (const __nv_bfloat16 *)qkv, NQKV, H, H + KV, rope_angles, d_slot,
-                                      k_base, v_base, d_bt, d_total, M, QH, KVH, HD, pool->block_size,
-                                      pool->max_blocks_per_seq, max_total, st)) {
+        // RoPE on q and k (position = cached length), KV write and attention over cached + 1 tokens: one launch ...
+        bool ok = !attn_scalar_forced() &&
+                  launch_paged_decode_split((__nv_bfloat16 *)att, H, (const __nv_bfloat16 *)qkv, NQKV, H, H + KV, rope_angles, d_slot,
+                                            k_base, v_base, d_bt, d_total, M, QH, KVH, HD, pool->block_size,
+                                            pool->max_blocks_per_seq, max_total, st, early_cache, o_q ? aq : nullptr,
+                                            o_q ? asf : nullptr, R.o.input_scale);
+        if (ok && !o_q) {
             single_proj(hid, H, att, H, R.o, M, hid, scratch);
             glue += project_mlp(R, hid, B, M, H, F, st);
             note_launches(glue + 1);
             continue;
         }
-        // RoPE on q and k in place (position = cached length), KV write, attention over cached + 1 tokens
-        if (launch_rope_qk_cache((__nv_bfloat16 *)qkv, NQKV, H, H + KV, d_seq_lens, d_slot, k_base, v_base, M, QH, KVH, HD, st, rope_angles)) {
-            glue += 1;
-        } else {
-            launch_rope_single_token((__nv_bfloat16 *)qkv, NQKV, 0, d_seq_lens, M, QH, HD, st);
-            launch_rope_single_token((__nv_bfloat16 *)qkv, NQKV, H, d_seq_lens, M, KVH, HD, st);
-            launch_reshape_and_cache(k_base, v_base, (const __nv_bfloat16 *)qkv + H, NQKV,
-                                     (const __nv_bfloat16 *)qkv + H + KV, NQKV, d_slot, M, KVH, HD, pool->block_size, st);
-            glue += 3;
+        // ... or, in layouts that one does not take, one each
+        if (!ok) {
+            if (launch_rope_qk_cache((__nv_bfloat16 *)qkv, NQKV, H, H + KV, d_seq_lens, d_slot, k_base, v_base, M, QH, KVH, HD, st, rope_angles)) {
+                glue += 1;
+            } else {
+                launch_rope_single_token((__nv_bfloat16 *)qkv, NQKV, 0, d_seq_lens, M, QH, HD, st);
+                launch_rope_single_token((__nv_bfloat16 *)qkv, NQKV, H, d_seq_lens, M, KVH, HD, st);
+                launch_reshape_and_cache(k_base, v_base, (const __nv_bfloat16 *)qkv + H, NQKV,
+                                         (const __nv_bfloat16 *)qkv + H + KV, NQKV, d_slot, M, KVH, HD, pool->block_size, st);
+                glue += 3;
+            }
+            if (o_q)
+                ok = launch_paged_decode_attention_mma((__nv_bfloat16 *)att, H, (const __nv_bfloat16 *)qkv, NQKV, k_base, v_base,
+                                                       d_bt, d_total, M, QH, KVH, HD, pool->block_size, pool->max_blocks_per_seq,
+                                                       st, aq, asf, R.o.input_scale);
         }
-        bool ok = false;
-        if (o_q)
-            ok = launch_paged_decode_attention_mma((__nv_bfloat16 *)att, H, (const __nv_bfloat16 *)qkv, NQKV, k_base, v_base, d_bt,
-                                                   d_total, M, QH, KVH, HD, pool->block_size, pool->max_blocks_per_seq, st, aq,
-                                                   asf, R.o.input_scale);
         if (ok && tail &&
             launch_layer_tail(R, l + 1 < L ? &refs.layers[l + 1] : nullptr, hid, B, gq, gsf, tail_counter, tail_base, M, H, KV, F, st)) {
             have_qkv = l + 1 < L;

@@ -69,7 +69,7 @@ __global__ void __launch_bounds__(kCgThreads, 2) cluster_gemm_kernel(const __gri
     const int row0 = silu ? wt * 64 : wt * 128;
     col0 += row0;
 
-    pdl_launch_dependents();
+    if (!p.late_trigger) pdl_launch_dependents();
     if (threadIdx.x == 0) {
         for (int s = 0; s < S; ++s) {
             mbar_init(full(s), 1);
@@ -106,6 +106,7 @@ __global__ void __launch_bounds__(kCgThreads, 2) cluster_gemm_kernel(const __gri
         for (int kb = 0; kb < pre; ++kb)
             if (leader) load_w(kb, kb);
         pdl_wait();
+        if (p.late_trigger) pdl_launch_dependents();
         int s = 0;
         uint32_t ph = 1;
         for (int kb = 0; kb < n_kb; ++kb) {

@@ -20,6 +20,7 @@ struct alignas(64) ClusterGemmParams {
     const __nv_bfloat16 *residual, *bias;
     int ldo;
     int early_weights;                  // 1: nothing still running writes the weights, load them before the dependency wait
+    int late_trigger;                   // 1: signal the dependents after the dependency wait
     int *status;
     // filled by choose_cluster_gemm
     int n_tok, token_tiles, splits, stages, w_tiles;

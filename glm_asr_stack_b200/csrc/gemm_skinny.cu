@@ -20,6 +20,8 @@
 //     multiplies the fp32 sums.  W4A4 rounds x through the activation quantiser instead: e2m1 * e4m3 is exact in bf16
 //     and the products are exact in fp32, so the result is the block-scaled MMA's up to the order of the sum;
 //   * the eight partial sums meet in shared memory, fixed order.
+// Asking for a warp's activations of several K chunks at once (two or three, 124 - 128 registers) made a decode step of one
+// sequence slower, 1106 against 1029 us, and so did three of these CTAs per SM at 80 registers (1076 against 999).
 // From 17 rows the tokens' operand no longer fits the registers beside the accumulators and the bf16 copies on the cluster
 // GEMM are faster (19 sequences: 1.96 against 2.33 ms a step).
 // Bound: instruction issue of the dequantisation (five instructions per two weights; 1.8 us for gate|up) and the fixed
@@ -139,7 +141,7 @@ __global__ void __launch_bounds__(kThreadsSk, 2) skinny_linear_kernel(const __gr
     const int u_end = min(p.units, u0 + p.units_per_cta);
     const int rounds = (u_end - u0 + p.units_per_group - 1) / p.units_per_group;
 
-    pdl_launch_dependents();
+    if (!p.late_trigger) pdl_launch_dependents();
     if (threadIdx.x == 0) {
         mbar_init(bars, 1);
         mbar_init(bars + 8, 1);
@@ -177,6 +179,7 @@ __global__ void __launch_bounds__(kThreadsSk, 2) skinny_linear_kernel(const __gr
     if (!p.early_weights) pdl_wait();
     for (int r = 0; r < p.groups && r < rounds; ++r) issue_round(r);
     if (p.early_weights) pdl_wait();
+    if (p.late_trigger) pdl_launch_dependents();
 
     const int chunks = p.K >> 7;
     float ss[NT];

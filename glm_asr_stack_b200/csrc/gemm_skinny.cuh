@@ -26,6 +26,7 @@ struct SkinnyParams {
     const __nv_bfloat16 *bias;
     int ldo;
     int early_weights;                  // 1: nothing still running writes the weights, load them before the dependency wait
+    int late_trigger;                   // 1: signal the dependents after the dependency wait
     int *status;
     // filled by the launcher
     int units, units_per_cta, units_per_group, groups, pass_tiles;

@@ -332,13 +332,15 @@ bool launch_paged_decode_attention_mma(__nv_bfloat16 *out, int ldo, const __nv_b
 }
 
 // --------------------------------------------------------------------------------------------
-// The same attention for a small batch, with what precedes it in a decode step folded in: RoPE on the new token's q and
+// The same attention with what precedes it in a decode step folded in: RoPE on the new token's q and
 // k heads, its K / V rows into the cache, attention over cached + 1 tokens.  A batch of a few sequences has kv_heads x
 // num_seqs blocks of work -- four CTAs for one sequence -- each a serial walk over the context, so the context of a
 // (sequence, kv head) is cut into `gridDim.x` contiguous shares, one CTA each, and the CTAs of a cluster merge their
 // partial results through distributed shared memory.  One sequence, 300 tokens: rope + cache and attention were two
 // launches of 3 + 9 us in the chain.  The new token's K / V row is put into the staged tile from the q|k|v buffer, so
-// the cache write is off the critical path.  16-token tiles inside one page (block_size % 16 == 0), head_dim 128.
+// the cache write is off the critical path; lengths, block table and cached rows are asked for while the projection still
+// runs (19 sequences: 13.3 -> 7.5 us).  A large batch takes it unsplit, one launch less (256 sequences: 2606 -> 2588 us a step).
+// 16-token tiles inside one page (block_size % 16 == 0), head_dim 128.
 // --------------------------------------------------------------------------------------------
 __device__ __forceinline__ float ld_cluster_f32(uint32_t addr) {
     float v;
@@ -350,11 +352,12 @@ __global__ void __launch_bounds__(kWarps * 32) paged_decode_split_kernel(
     __nv_bfloat16 *__restrict__ out, int ldo, const __nv_bfloat16 *__restrict__ qkv, int ld, int k_col, int v_col,
     const float *__restrict__ angles, const int64_t *__restrict__ slot_mapping, __nv_bfloat16 *key_cache,
     __nv_bfloat16 *value_cache, const int *__restrict__ block_tables, const int *__restrict__ seq_lens, int num_kv_heads,
-    int group, int block_size, int max_blocks_per_seq, float scale) {
+    int group, int block_size, int max_blocks_per_seq, float scale, int early_cache, uint8_t *__restrict__ q_packed,
+    uint8_t *__restrict__ q_sf, int q_sf_chunks, float q_inv_in) {
     extern __shared__ __align__(1024) uint8_t smem[];
     __shared__ float merged[8 * 130];           // this CTA's result per head: max, sum, 128 accumulators
     pdl_launch_dependents();
-    pdl_wait();
+    if (!early_cache) pdl_wait();
     const int split = blockIdx.x, splits = gridDim.x, kv_head = blockIdx.y, seq = blockIdx.z;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, tq = lane & 3;
@@ -400,6 +403,7 @@ __global__ void __launch_bounds__(kWarps * 32) paged_decode_split_kernel(
         if (i < my_tiles) load_tile(i);
         cp_async_commit();
     }
+    if (early_cache) pdl_wait();        // up to here: lengths, block table and cached rows, none of them the q|k|v projection's
 
     // q fragments, rotated in registers: a lane holds dims d and d + 64 of its head (k steps ks and ks + 4)
     uint32_t qa[8][2];
@@ -532,7 +536,9 @@ __global__ void __launch_bounds__(kWarps * 32) paged_decode_split_kernel(
             den += e * pw[1];
         }
         if (splits == 1) {
-            out[(size_t)seq * ldo + (size_t)(q_head0 + h) * 128 + d] = __float2bfloat16(num / (den + 1e-9f));
+            const __nv_bfloat16 v = __float2bfloat16(num / (den + 1e-9f));
+            if (q_packed != nullptr) merged[h * 128 + d] = __bfloat162float(v);
+            else out[(size_t)seq * ldo + (size_t)(q_head0 + h) * 128 + d] = v;
         } else {
             merged[h * kPart + 2 + d] = num;
             if (d == 0) {
@@ -541,7 +547,25 @@ __global__ void __launch_bounds__(kWarps * 32) paged_decode_split_kernel(
             }
         }
     }
-    if (splits == 1) return;
+    if (splits == 1) {
+        if (q_packed == nullptr) return;
+        // finished heads through the activation quantiser
+        __syncthreads();
+        const int hidden = num_kv_heads * group * 128;
+        for (int task = threadIdx.x; task < group * 8; task += blockDim.x) {
+            const int h = task >> 3, b = task & 7;
+            float v[16];
+#pragma unroll
+            for (int j = 0; j < 16; ++j) v[j] = merged[h * 128 + b * 16 + j];
+            uint32_t lo, hi;
+            const uint32_t sf = quantize_block16(v, q_inv_in, lo, hi);
+            const int col = (q_head0 + h) * 128 + b * 16;
+            *reinterpret_cast<uint2 *>(q_packed + (size_t)seq * (hidden / 2) + (col >> 1)) = make_uint2(lo, hi);
+            const int kb = col >> 4, rem = seq & 127;
+            q_sf[((((size_t)(seq >> 7) * q_sf_chunks + (kb >> 2)) * 32 + (rem & 31)) * 4 + (rem >> 5)) * 4 + (kb & 3)] = (uint8_t)sf;
+        }
+        return;
+    }
     cluster_sync_all();
     const uint32_t base = smem_u32(merged);
     for (int idx = split * (int)blockDim.x + threadIdx.x; idx < group * 128; idx += splits * (int)blockDim.x) {
@@ -575,16 +599,21 @@ bool launch_paged_decode_split(__nv_bfloat16 *out, int ldo, const __nv_bfloat16 
                                const float *angles, const int64_t *slot_mapping, __nv_bfloat16 *key_cache,
                                __nv_bfloat16 *value_cache, const int *block_tables, const int *seq_lens, int num_seqs,
                                int num_q_heads, int num_kv_heads, int head_dim, int block_size, int max_blocks_per_seq,
-                               int max_len, cudaStream_t st) {
+                               int max_len, cudaStream_t st, bool early_cache, uint8_t *q_packed, uint8_t *q_sf, float q_input_scale) {
     if (head_dim != 128 || num_kv_heads <= 0 || num_q_heads % num_kv_heads != 0 || num_seqs <= 0 || angles == nullptr) return false;
     const int group = num_q_heads / num_kv_heads;
     if (group > 8 || (ld % 8) != 0 || (k_col % 8) != 0 || (v_col % 8) != 0 || (block_size % kTile) != 0) return false;
     if ((((uintptr_t)key_cache | (uintptr_t)value_cache | (uintptr_t)qkv) & 15) != 0) return false;
-    // three 64 KB CTAs fit an SM: up to 444 in one wave, at least two tiles for every CTA
+    if (q_packed != nullptr && (q_sf == nullptr || !(q_input_scale > 0.0f) || (((uintptr_t)q_packed) & 7) != 0)) return false;
+    // unsplit on a chip that it leaves half empty, the serial walk with RoPE in front of it is the longer way round: a W4A4
+    // step of 1 / 9 sequences, 16 query and 4 kv heads, takes 1745 / 1823 us with it and 1710 / 1788 us with two launches,
+    // of 19 sequences 1813 and 1817 us, of 40 / 100 sequences 1807 / 1896 and 1857 / 1963 us
+    if (q_packed != nullptr && num_seqs * num_kv_heads <= 74) return false;
+    // three 64 KB CTAs fit an SM: up to 444 in one wave, at least two tiles for every CTA.  A result that is quantised is not
+    // split: another order of its sums moves values across e2m1 rounding boundaries, and a chain of such layers amplifies it.
     const int tiles = (max_len + kTile - 1) / kTile;
     int splits = 1;
-    while (splits < 8 && num_seqs * num_kv_heads * splits * 2 <= 444 && tiles >= splits * 4) splits *= 2;
-    if (splits == 1 && num_seqs * num_kv_heads > 222) return false;      // enough work without a split: the two-launch path
+    while (q_packed == nullptr && splits < 8 && num_seqs * num_kv_heads * splits * 2 <= 444 && tiles >= splits * 4) splits *= 2;
     static bool configured = false;
     if (!configured) {
         if (cudaFuncSetAttribute(paged_decode_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kAttnSmem) != cudaSuccess)
@@ -609,7 +638,8 @@ bool launch_paged_decode_split(__nv_bfloat16 *out, int ldo, const __nv_bfloat16 
     cfg.numAttrs = pdl_enabled() ? 2 : 1;
     return cudaLaunchKernelEx(&cfg, paged_decode_split_kernel, out, ldo, qkv, ld, k_col, v_col, angles, slot_mapping, key_cache,
                               value_cache, block_tables, seq_lens, num_kv_heads, group, block_size, max_blocks_per_seq,
-                              1.0f / sqrtf((float)head_dim)) == cudaSuccess;
+                              1.0f / sqrtf((float)head_dim), early_cache && pdl_enabled() ? 1 : 0, q_packed, q_sf,
+                              num_q_heads * head_dim / 64, q_packed != nullptr ? 1.0f / q_input_scale : 0.0f) == cudaSuccess;
 }
 
 }  // namespace glmasr

@@ -75,6 +75,15 @@ struct SettledWeights {
     bool before;
 };
 bool weights_settled();
+// In its scope a GEMM that can do so signals its dependents only after its own pdl_wait(): when the kernel behind it
+// starts, everything in FRONT of the GEMM has completed, and that kernel may read such results before its pdl_wait().
+struct LateTrigger {
+    LateTrigger();
+    ~LateTrigger();
+};
+bool late_trigger_asked();
+void note_late_trigger(bool taken);
+bool late_trigger_taken();          // by the last GEMM launched
 
 #ifdef __CUDACC__
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }

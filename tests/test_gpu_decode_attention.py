@@ -1,0 +1,80 @@
+"""RoPE + cache write + attention of a decode step as one launch, where its split of the context can go wrong: context
+lengths around the 16-token tiles and the shares of a cluster, sequences of one batch that leave shares empty, batches
+too large to be split, and the result handed on as bf16 or as the quantised operand of the o projection.  Checked
+through decoder_decode_step_batched on the small model against the oracle, with the bounds of its other driver cases."""
+import ctypes
+import os
+import subprocess
+import sys
+
+import numpy as np
+import pytest
+import torch
+
+import decoder_oracle as do
+import fp4_oracle as o
+import test_gpu_decoder as tgd
+from conftest import ROOT
+from gpu_util import REL_TOL_VS_ORACLE, bits_of, to_dev_bf16
+
+pytestmark = pytest.mark.gpu
+
+CONTEXTS = {
+    "one-new": [0],                                        # nothing cached: the new token attends to itself
+    "one-tile-edge": [15],
+    "one-split": [511],                                    # 32 tiles over the largest cluster
+    "one-split-ragged": [272],                             # 18 tiles: the last shares are short
+    "uneven": [0, 1, 15, 16, 17, 62, 63, 64, 450],         # most shares of the short sequences are empty
+    "few": [(11 * i) % 70 for i in range(74)],             # the last batch whose quantised result comes from two launches
+    "many": [(11 * i) % 70 for i in range(75)],            # ... and the first from one
+    "unsplit": [(7 * i) % 83 for i in range(230)],         # more CTAs than a split could use
+}
+
+
+def run_contexts(mode):
+    from glm_asr_stack_b200 import engine, ops
+    rng = np.random.default_rng(31)
+    ws, cfg, layers, fn, (H, F, QH, KVH, HD, L) = tgd.build_toy_model(rng, 700, "plain")
+    lin = tgd.oracle_linears(layers, mode)
+    bs, max_blocks = 16, 33
+    errs = {}
+    for name, ctx in CONTEXTS.items():
+        cached, n = np.array(ctx, np.int32), len(ctx)
+        num_blocks = sum(c // bs + 1 for c in ctx) + 3
+        pool = engine.KVPool(num_blocks, bs, L, KVH, HD, max_seqs=n, max_blocks_per_seq=max_blocks)
+        perm = rng.permutation(num_blocks).tolist()
+        tables = [[perm.pop() for _ in range(c // bs + 1)] for c in ctx]
+        bts = engine.BlockTables(pool, tables)
+        bt_np = np.full((n, max_blocks), -1, np.int32)
+        for i, t in enumerate(tables):
+            bt_np[i, :len(t)] = t
+        kc0 = tgd.rnd_bits(rng, (L, num_blocks * bs, KVH * HD))
+        vc0 = tgd.rnd_bits(rng, (L, num_blocks * bs, KVH * HD))
+        pool.k.copy_(to_dev_bf16(kc0).view(pool.k.shape))
+        pool.v.copy_(to_dev_bf16(vc0).view(pool.v.shape))
+        hidden = tgd.rnd_bits(rng, (n, H))
+        x = to_dev_bf16(hidden)
+        d_lens = torch.from_numpy(cached.copy()).cuda()
+        engine.decode_step(ws, cfg, pool, bts, x, d_lens, (ctypes.c_int * n)(*ctx))
+        torch.cuda.synchronize()
+        assert ops.status() == 0
+        slots = np.array([bt_np[i, c // bs] * bs + c % bs for i, c in enumerate(ctx)], np.int64)
+        kc, vc = [kc0[l].copy() for l in range(L)], [vc0[l].copy() for l in range(L)]
+        want = do.decode_step(hidden, layers, fn, kc, vc, bt_np, cached, slots, QH, KVH, HD, bs, lin)
+        errs[name] = o.rel_err(bits_of(x), want)
+        assert errs[name] <= REL_TOL_VS_ORACLE, (name, errs)
+        others = np.ones(num_blocks * bs, bool)
+        others[slots] = False                              # only the new token's rows are written
+        for l in range(L):
+            for dev, before in ((pool.k, kc0), (pool.v, vc0)):
+                assert np.array_equal(bits_of(dev[l].reshape(num_blocks * bs, -1))[others], before[l][others]), (name, l)
+    return errs
+
+
+@pytest.mark.parametrize("mode", ["w4a16", "all_w4a4"])
+def test_decode_attention_contexts(mode):
+    code = ("import sys; sys.path[:0]=[%r,%r,%r]; import test_gpu_decode_attention as t; print('RESULT', t.run_contexts(%r))"
+            % (ROOT, os.path.join(ROOT, "oracle"), os.path.join(ROOT, "tests"), mode))
+    r = subprocess.run([sys.executable, "-c", code], env=dict(os.environ, **tgd.MODE_ENV[mode]), capture_output=True,
+                       text=True, timeout=600)
+    assert r.returncode == 0 and "RESULT" in r.stdout, r.stdout[-4000:] + r.stderr[-4000:]
