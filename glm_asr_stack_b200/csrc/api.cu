@@ -573,7 +573,11 @@ static int route_rows(const FusedArgs &a) { return a.M > g_route_rows ? a.M : g_
 
 static bool skinny_eligible(const FusedArgs &a) {
     if (a.mode == GEMM_BF16 || a.pre != nullptr || a.xq != nullptr || a.q_out != nullptr) return false;
-    if (a.mode == GEMM_W4A4 && (route_rows(a) > 8 || a.num_w != 1 || a.epi != EPI_STORE)) return false;
+    // W4A4: every CTA quantises the rows for itself and dequantises what the block-scaled MMA takes as it lies, so only the
+    // fewer launches count.  One row, us, weights not in L2, this kernel against the other route: [512, 2048] 8.2 / 14.0 (4 rows
+    // 7.8 / 8.7), [2048, 2048] 8.5 / 11.2 (4 rows 7.9 / 8.7), [6144, 2048] 10.6 / 9.0, [2048, 6144] 20.4 / 11.1,
+    // [59264, 2048] 57.0 / 18.9
+    if (a.mode == GEMM_W4A4 && (route_rows(a) > 8 || a.num_w != 1 || a.epi != EPI_STORE || a.w[0].N > 2048 || a.K > 2048)) return false;
     int rows[kMaxSegments];
     for (int i = 0; i < a.num_w; ++i) rows[i] = a.w[i].N;
     return skinny_covers(route_rows(a), a.K, rows, a.num_w, a.epi);
@@ -708,7 +712,7 @@ static int run_fused(const FusedArgs &a) {
     }
 
     // A handful of rows: the few-row kernel reads the packed weights as they are.  W4A16 takes it up to its 16 rows.  A
-    // single W4A4 linear does up to 8 (every CTA quantises the rows for itself); fused W4A4 projections and quantised
+    // single W4A4 linear of a small matrix does up to 8 (every CTA quantises the rows for itself); fused W4A4 projections and quantised
     // hand-overs, the parts of a chain, stay on the block-scaled MMA whose bits they share with the resident kernel.
     if (skinny_eligible(a)) return run_skinny(a);
 
