@@ -572,12 +572,7 @@ static const __nv_bfloat16 *resident_bf16_weight(const glmasr_fp4_weight &w, int
 static int route_rows(const FusedArgs &a) { return a.M > g_route_rows ? a.M : g_route_rows; }
 
 static bool skinny_eligible(const FusedArgs &a) {
-    if (a.mode == GEMM_BF16 || a.pre != nullptr || a.xq != nullptr || a.q_out != nullptr) return false;
-    // W4A4: every CTA quantises the rows for itself and dequantises what the block-scaled MMA takes as it lies, so only the
-    // fewer launches count.  One row, us, weights not in L2, this kernel against the other route: [512, 2048] 8.2 / 14.0 (4 rows
-    // 7.8 / 8.7), [2048, 2048] 8.5 / 11.2 (4 rows 7.9 / 8.7), [6144, 2048] 10.6 / 9.0, [2048, 6144] 20.4 / 11.1,
-    // [59264, 2048] 57.0 / 18.9
-    if (a.mode == GEMM_W4A4 && (route_rows(a) > 8 || a.num_w != 1 || a.epi != EPI_STORE || a.w[0].N > 2048 || a.K > 2048)) return false;
+    if (a.mode != GEMM_W4A16 || a.pre != nullptr || a.q_out != nullptr) return false;
     int rows[kMaxSegments];
     for (int i = 0; i < a.num_w; ++i) rows[i] = a.w[i].N;
     return skinny_covers(route_rows(a), a.K, rows, a.num_w, a.epi);
@@ -592,13 +587,12 @@ static int run_skinny(const FusedArgs &a, const __nv_bfloat16 *norm_w = nullptr,
     p.K = a.K;
     p.norm_w = norm_w;
     p.eps = eps;
-    p.inv_in = a.mode == GEMM_W4A4 ? 1.0f / a.input_scale : 0.0f;
     double n_rows = 0.0;
     for (int i = 0; i < a.num_w; ++i) {
         p.w[i] = a.w[i].w_packed;
         p.ws[i] = a.w[i].w_scales;
         p.seg_rows[i] = a.w[i].N;
-        p.alpha[i] = a.mode == GEMM_W4A4 ? a.input_scale * a.w[i].w_global_scale : a.w[i].w_global_scale;
+        p.alpha[i] = a.w[i].w_global_scale;
         n_rows += a.w[i].N;
     }
     p.num_segs = a.num_w;
@@ -607,7 +601,7 @@ static int run_skinny(const FusedArgs &a, const __nv_bfloat16 *norm_w = nullptr,
     p.residual = a.residual;
     p.bias = a.bias;
     p.ldo = a.ldo;
-    p.early_weights = a.mode == GEMM_W4A4 || weights_settled() ? 1 : 0;
+    p.early_weights = weights_settled() ? 1 : 0;
     p.status = device_status_word();
     profile_bracket_begin(2.0 * a.M * n_rows * a.K, 0.5625 * n_rows * a.K + 2.0 * a.M * (a.K + total_out_cols(a)));
     p.late_trigger = late_trigger_asked() ? 1 : 0;
@@ -711,9 +705,7 @@ static int run_fused(const FusedArgs &a) {
         return run_simt(a);
     }
 
-    // A handful of rows: the few-row kernel reads the packed weights as they are.  W4A16 takes it up to its 16 rows.  A
-    // single W4A4 linear of a small matrix does up to 8 (every CTA quantises the rows for itself); fused W4A4 projections and quantised
-    // hand-overs, the parts of a chain, stay on the block-scaled MMA whose bits they share with the resident kernel.
+    // W4A16 with a handful of rows: the few-row kernel reads the packed weights as they are.
     if (skinny_eligible(a)) return run_skinny(a);
 
     // W4A16 on resident bf16 copies of the weights (made on first use, within the budget): the bf16 GEMM streams

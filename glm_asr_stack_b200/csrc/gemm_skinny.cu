@@ -1,4 +1,4 @@
-// W4A16 / W4A4 linear for a handful of rows (decode of a few sequences).
+// W4A16 linear for a handful of rows (decode of a few sequences).
 //
 // With M <= 16 rows the tcgen05 kernels leave most of the chip idle: a 2048-column projection has sixteen 128-wide
 // tiles, and each of those CTAs pulls its whole K range through one ring at the ~100 GB/s one SM gets (down projection,
@@ -17,11 +17,12 @@
 //     (subnormals included), one packed multiply by scale * 2^112 gives value * scale * 2^-14 exactly, and 2^14 goes into
 //     the per-tensor factor;
 //   * RMSNorm of the input is folded in: x * w is rounded to bf16 as the operand, 1 / rms (from the same registers)
-//     multiplies the fp32 sums.  W4A4 rounds x through the activation quantiser instead: e2m1 * e4m3 is exact in bf16
-//     and the products are exact in fp32, so the result is the block-scaled MMA's up to the order of the sum;
+//     multiplies the fp32 sums;
 //   * the eight partial sums meet in shared memory, fixed order.
 // Asking for a warp's activations of several K chunks at once (two or three, 124 - 128 registers) made a decode step of one
 // sequence slower, 1106 against 1029 us, and so did three of these CTAs per SM at 80 registers (1076 against 999).
+// W4A4 stays on the block-scaled MMA: with the quantiser folded in here too (every CTA rounds the rows for itself) one row of
+// [2048, 2048] took 8.5 us on the device against 7.2 for quantiser and MMA.
 // From 17 rows the tokens' operand no longer fits the registers beside the accumulators and the bf16 copies on the cluster
 // GEMM are faster (19 sequences: 1.96 against 2.33 ms a step).
 // Bound: instruction issue of the dequantisation (five instructions per two weights; 1.8 us for gate|up) and the fixed
@@ -30,7 +31,6 @@
 
 #include <cuda_bf16.h>
 
-#include "fp4_format.cuh"
 #include "gemm_umma.cuh"
 #include "ptx.cuh"
 #include "runtime.cuh"
@@ -83,7 +83,7 @@ __device__ __forceinline__ void mma_16816(float (&d)[4], uint32_t a0, uint32_t a
                  : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-enum SkinnySource : int { SK_PLAIN = 0, SK_NORM = 1, SK_QUANT = 2 };
+enum SkinnySource : int { SK_PLAIN = 0, SK_NORM = 1 };
 
 // One 8-element word pair order: elements 0..7 of `v` (four bf16x2 words) as the pairs (0,4) (1,5) (2,6) (3,7).
 __device__ __forceinline__ void permute8(const uint4 &v, uint32_t (&o)[4]) {
@@ -91,34 +91,6 @@ __device__ __forceinline__ void permute8(const uint4 &v, uint32_t (&o)[4]) {
     o[1] = __byte_perm(v.x, v.z, 0x7632);
     o[2] = __byte_perm(v.y, v.w, 0x5410);
     o[3] = __byte_perm(v.y, v.w, 0x7632);
-}
-
-// Two 16-element blocks (32 elements, 16 words) through the quantiser and back: each block becomes code * scale in bf16.
-__device__ __forceinline__ void fake_quantise(uint4 (&v)[4], float inv_in) {
-#pragma unroll
-    for (int b = 0; b < 2; ++b) {
-        float f[16];
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const uint32_t w[4] = {v[2 * b + h].x, v[2 * b + h].y, v[2 * b + h].z, v[2 * b + h].w};
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                f[8 * h + 2 * j] = __uint_as_float(w[j] << 16);
-                f[8 * h + 2 * j + 1] = __uint_as_float(w[j] & 0xFFFF0000u);
-            }
-        }
-        uint32_t lo, hi;
-        const float s = e4m3_to_float_ref(quantize_block16(f, inv_in, lo, hi));
-        uint32_t o[8];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const uint32_t byte = ((j < 4 ? lo : hi) >> (8 * (j & 3))) & 0xFFu;
-            const __nv_bfloat162 p = __floats2bfloat162_rn(e2m1_to_float(byte & 15u) * s, e2m1_to_float(byte >> 4) * s);
-            o[j] = *reinterpret_cast<const uint32_t *>(&p);
-        }
-        v[2 * b] = make_uint4(o[0], o[1], o[2], o[3]);
-        v[2 * b + 1] = make_uint4(o[4], o[5], o[6], o[7]);
-    }
 }
 
 template <int NT, int SRC>
@@ -227,7 +199,6 @@ __global__ void __launch_bounds__(kThreadsSk, 2) skinny_linear_kernel(const __gr
                                               mul_bf16x2(v[j].w, w4.w));
                         }
                     }
-                    if (SRC == SK_QUANT) fake_quantise(v, p.inv_in);
 #pragma unroll
                     for (int j = 0; j < 4; ++j) {
                         uint32_t o[4];
@@ -343,11 +314,9 @@ bool skinny_covers(int M, int K, const int *seg_rows, int num_segs, int epi) {
 
 template <int NT>
 static cudaError_t launch_nt(const SkinnyParams &p, int grid, size_t smem, cudaStream_t st) {
-    void (*kernel)(SkinnyParams) = p.norm_w != nullptr ? skinny_linear_kernel<NT, SK_NORM>
-                                   : p.inv_in > 0.0f   ? skinny_linear_kernel<NT, SK_QUANT>
-                                                       : skinny_linear_kernel<NT, SK_PLAIN>;
-    static bool ready[3] = {false, false, false};
-    const int which = p.norm_w != nullptr ? SK_NORM : (p.inv_in > 0.0f ? SK_QUANT : SK_PLAIN);
+    void (*kernel)(SkinnyParams) = p.norm_w != nullptr ? skinny_linear_kernel<NT, SK_NORM> : skinny_linear_kernel<NT, SK_PLAIN>;
+    static bool ready[2] = {false, false};
+    const int which = p.norm_w != nullptr ? SK_NORM : SK_PLAIN;
     if (!ready[which]) {
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
         if (e == cudaSuccess)

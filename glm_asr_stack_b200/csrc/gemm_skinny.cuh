@@ -14,7 +14,6 @@ struct SkinnyParams {
     int ldx, M, K;
     const __nv_bfloat16 *norm_w;        // not NULL: x is RMS-normalised with this weight first (eps below)
     float eps;
-    float inv_in;                       // > 0: x goes through the activation quantiser (1 / input_scale) first: W4A4
     const uint8_t *w[3];                // packed e2m1 [N_s, K/2]
     const uint8_t *ws[3];               // e4m3 [N_s, K/16]
     float alpha[3];                     // per-tensor factor of segment s
