@@ -49,7 +49,8 @@ bool launch_paged_decode_attention_mma(__nv_bfloat16 *out, int ldo, const __nv_b
 // RoPE + cache write + attention of a decode batch as one launch, the context of a small batch cut over clusters; angles as
 // launch_rope_angles writes them, max_len = the longest context (tokens attended).  early_cache: everything but the q|k|v
 // projection in front has completed when this kernel starts (LateTrigger).  With q_packed the result is written as the
-// quantised operand of the o projection instead of bf16.  False when the layout is not covered (nothing launched).
+// quantised operand of the o projection instead of bf16.  No row may attend to a token that another row writes (step_pages.h).
+// False when the layout is not covered (nothing launched).
 bool launch_paged_decode_split(__nv_bfloat16 *out, int ldo, const __nv_bfloat16 *qkv, int ld, int k_col, int v_col,
                                const float *angles, const int64_t *slot_mapping, __nv_bfloat16 *key_cache,
                                __nv_bfloat16 *value_cache, const int *block_tables, const int *seq_lens, int num_seqs,

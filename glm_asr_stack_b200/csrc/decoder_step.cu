@@ -28,6 +28,7 @@
 #include "decode_tail.cuh"
 #include "decoder_ops.cuh"
 #include "runtime.cuh"
+#include "step_pages.h"
 
 namespace glmasr {
 int fp4_linear_w4a4_prequantized(uint16_t *out, int ldo, const uint8_t *xq, const uint8_t *xq_sf,
@@ -802,6 +803,7 @@ extern "C" void decoder_decode_step_batched(void *handle, const void *ws_v, uint
                      "decoder_decode_step_batched: invalid seq index %d for batch row %d", h_rows[s], s);
         if (query_ptrs[s] != query_ptrs[0] + (size_t)s * H) contiguous = false;
     }
+    const bool rows_independent = !rows_share_new_pages(bts, h_seq_lens, M, pool->block_size);
 
     uint16_t *hid = (uint16_t *)workspace_slot(WS_D_HID, (size_t)M * H * 2);
     uint16_t *nrm = (uint16_t *)workspace_slot(WS_D_NORM, (size_t)M * H * 2);
@@ -878,7 +880,7 @@ extern "C" void decoder_decode_step_batched(void *handle, const void *ws_v, uint
         // attention writes the o projection's quantised operand itself when that projection runs in W4A4
         const bool o_q = takes_quantised_input(R.o) && R.o.K == H && !attn_scalar_forced();
         // RoPE on q and k (position = cached length), KV write and attention over cached + 1 tokens: one launch ...
-        bool ok = !attn_scalar_forced() &&
+        bool ok = rows_independent && !attn_scalar_forced() &&
                   launch_paged_decode_split((__nv_bfloat16 *)att, H, (const __nv_bfloat16 *)qkv, NQKV, H, H + KV, rope_angles, d_slot,
                                             k_base, v_base, d_bt, d_total, M, QH, KVH, HD, pool->block_size,
                                             pool->max_blocks_per_seq, max_total, st, early_cache, o_q ? aq : nullptr,
@@ -889,7 +891,7 @@ extern "C" void decoder_decode_step_batched(void *handle, const void *ws_v, uint
             note_launches(glue + 1);
             continue;
         }
-        // ... or, in layouts that one does not take, one each
+        // ... or, in layouts that one does not take and where rows read what others of the step write, one each
         if (!ok) {
             if (launch_rope_qk_cache((__nv_bfloat16 *)qkv, NQKV, H, H + KV, d_seq_lens, d_slot, k_base, v_base, M, QH, KVH, HD, st, rope_angles)) {
                 glue += 1;

@@ -78,3 +78,58 @@ def test_decode_attention_contexts(mode):
     r = subprocess.run([sys.executable, "-c", code], env=dict(os.environ, **tgd.MODE_ENV[mode]), capture_output=True,
                        text=True, timeout=600)
     assert r.returncode == 0 and "RESULT" in r.stdout, r.stdout[-4000:] + r.stderr[-4000:]
+
+
+# rows that attend to a token another row of the same step writes: (tokens in the cache, pages of row i are those of row j)
+SHARED = {
+    "consecutive": ([37, 38], {1: 0}),                     # two tokens of one sequence in one step
+    "consecutive-over-a-page": ([15, 16, 200], {1: 0}),
+    "same-slot-twice": ([20, 20, 50], {1: 0}),             # a batch padded with a copy of a row
+    "run-of-many": ([40 + i for i in range(24)] + [9], {i: 0 for i in range(1, 24)}),
+}
+
+
+def run_shared(mode):
+    from glm_asr_stack_b200 import engine, ops
+    rng = np.random.default_rng(37)
+    ws, cfg, layers, fn, (H, F, QH, KVH, HD, L) = tgd.build_toy_model(rng, 900, "plain")
+    lin = tgd.oracle_linears(layers, mode)
+    bs, max_blocks, num_blocks = 16, 20, 64
+    errs = {}
+    for name, (ctx, same) in SHARED.items():
+        n, cached = len(ctx), np.array(ctx, np.int32)
+        perm = rng.permutation(num_blocks).tolist()
+        need = [max(c for j, c in enumerate(ctx) if same.get(j, j) == i) // bs + 1 if i not in same else 0 for i in range(n)]
+        own = [[perm.pop() for _ in range(b)] for b in need]
+        tables = [own[same.get(i, i)] for i in range(n)]
+        kc0, vc0 = (tgd.rnd_bits(rng, (L, num_blocks * bs, KVH * HD)) for _ in range(2))
+        hidden = tgd.rnd_bits(rng, (n, H))
+        if name == "same-slot-twice":
+            hidden[1] = hidden[0]
+        bt_np = np.full((n, max_blocks), -1, np.int32)
+        for i, t in enumerate(tables):
+            bt_np[i, :len(t)] = t
+        slots = np.array([bt_np[i, c // bs] * bs + c % bs for i, c in enumerate(ctx)], np.int64)
+        kc, vc = [kc0[l].copy() for l in range(L)], [vc0[l].copy() for l in range(L)]
+        want = do.decode_step(hidden, layers, fn, kc, vc, bt_np, cached, slots, QH, KVH, HD, bs, lin)
+        for _ in range(5):
+            pool = engine.KVPool(num_blocks, bs, L, KVH, HD, max_seqs=n, max_blocks_per_seq=max_blocks)
+            bts = engine.BlockTables(pool, tables)
+            pool.k.copy_(to_dev_bf16(kc0).view(pool.k.shape))
+            pool.v.copy_(to_dev_bf16(vc0).view(pool.v.shape))
+            x = to_dev_bf16(hidden)
+            engine.decode_step(ws, cfg, pool, bts, x, torch.from_numpy(cached.copy()).cuda(), (ctypes.c_int * n)(*ctx))
+            torch.cuda.synchronize()
+            assert ops.status() == 0
+            errs[name] = o.rel_err(bits_of(x), want)
+            assert errs[name] <= REL_TOL_VS_ORACLE, (name, errs)
+    return errs
+
+
+@pytest.mark.parametrize("mode", ["w4a16", "all_w4a4"])
+def test_rows_that_read_what_other_rows_write(mode):
+    code = ("import sys; sys.path[:0]=[%r,%r,%r]; import test_gpu_decode_attention as t; print('RESULT', t.run_shared(%r))"
+            % (ROOT, os.path.join(ROOT, "oracle"), os.path.join(ROOT, "tests"), mode))
+    r = subprocess.run([sys.executable, "-c", code], env=dict(os.environ, **tgd.MODE_ENV[mode]), capture_output=True,
+                       text=True, timeout=600)
+    assert r.returncode == 0 and "RESULT" in r.stdout, r.stdout[-4000:] + r.stderr[-4000:]
