@@ -30,7 +30,6 @@ static int *g_status = nullptr;
 static long long g_launches = 0;
 // Per-device facts and one-time set-up (the large shared-memory opt-in is an attribute of the kernel ON a
 // device): indexed by the current device, so a process that drives several GPUs sets each one up.
-static constexpr int kMaxDevices = 64;
 static int g_num_sms[kMaxDevices] = {0};
 static bool g_umma_ready[kMaxDevices] = {false};
 static bool g_pair16_ready[kMaxDevices] = {false};

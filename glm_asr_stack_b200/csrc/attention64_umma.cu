@@ -355,11 +355,9 @@ __global__ void __launch_bounds__(THREADS64, CTAS_PER_SM) attention64_umma_kerne
 bool launch_attention64_umma(__nv_bfloat16 *out, int ldo, const __nv_bfloat16 *q, int ldq, const __nv_bfloat16 *k, int ldk,
                              const __nv_bfloat16 *v, int ldv, const int *seq_offsets, const int *seq_lens, int num_seqs,
                              int max_seq_len, int total_tokens, int num_q_heads, int num_kv_heads, bool causal, cudaStream_t st) {
-    static bool configured = false;
-    if (!configured) {
-        if (cudaFuncSetAttribute(attention64_umma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM64) != cudaSuccess) return false;
-        configured = true;
-    }
+    static PerDevice<bool> configured;
+    if (once_per_device(configured, [] { return cudaFuncSetAttribute(attention64_umma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM64); }) != cudaSuccess)
+        return false;
     GLMASR_PREFER_MAX_SMEM(attention64_umma_kernel);
     Attn64Params p;
     memset(&p, 0, sizeof(p));

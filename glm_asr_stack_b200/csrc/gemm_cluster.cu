@@ -295,24 +295,29 @@ static ClusterGemmKernel cg_kernel(int splits) {
 }
 
 static cudaError_t cg_ready() {
-    static bool ready = false;
-    if (ready) return cudaSuccess;
-    for (int c : {1, 4, 8}) {
-        cudaError_t e = cudaFuncSetAttribute(cg_kernel(c), cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(cg_kernel(c), cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared);
-        if (e != cudaSuccess) return e;
-    }
-    ready = true;
-    return cudaSuccess;
+    static PerDevice<bool> ready;
+    return once_per_device(ready, [] {
+        for (int c : {1, 4, 8}) {
+            cudaError_t e = cudaFuncSetAttribute(cg_kernel(c), cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+            if (e == cudaSuccess)
+                e = cudaFuncSetAttribute(cg_kernel(c), cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared);
+            if (e != cudaSuccess) return e;
+        }
+        return cudaSuccess;
+    });
 }
 
 // Clusters of `splits` CTAs that the device holds at once at this shared-memory size (graphics processing clusters have
-// 16 to 20 SMs here, so it is less than 148 * 2 / splits); asked once per pair.
+// 16 to 20 SMs here, so it is less than 148 * 2 / splits), 0 when it holds none; asked once per pair and device.
 static int cg_max_clusters(int splits, size_t smem) {
-    static int known[9][16] = {{0}};
+    struct Known {
+        int n[9][16];               // 0: not asked yet, -1: none
+    };
+    static PerDevice<Known> known;
+    Known *k = known.here();
+    if (k == nullptr) return 0;
     const int slot = (int)(smem >> 14) & 15;
-    int &v = known[splits][slot];
+    int &v = k->n[splits][slot];
     if (v == 0) {
         cudaLaunchConfig_t cfg;
         cudaLaunchAttribute attr[2];
@@ -321,11 +326,11 @@ static int cg_max_clusters(int splits, size_t smem) {
         int n = 0;
         if (cudaOccupancyMaxActiveClusters(&n, cg_kernel(splits), &cfg) != cudaSuccess || n < 1) {
             (void)cudaGetLastError();
-            n = 1;
+            n = -1;
         }
         v = n;
     }
-    return v;
+    return v > 0 ? v : 0;
 }
 
 // Times in ns, fitted to launches of this kernel on a B200 (19 to 256 rows, K 1280 to 6144; within 15 %): a fixed 3.5 us,
@@ -347,6 +352,7 @@ double choose_cluster_gemm(ClusterGemmParams &p, int w_tiles) {
         for (int c = 1; c <= 8 && (c == 1 || c * 2 <= p.k_blocks); ++c) {
             const int clusters = w_tiles * tt;
             const int room = cg_max_clusters(c, smem);
+            if (room == 0) continue;
             const double waves = (clusters + room - 1) / room;
             const double share = clusters * c > 148 && smem <= 113 * 1024 ? 2.0 : 1.0;
             const int kb = (p.k_blocks + c - 1) / c;

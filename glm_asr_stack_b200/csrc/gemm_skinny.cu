@@ -315,15 +315,13 @@ bool skinny_covers(int M, int K, const int *seg_rows, int num_segs, int epi) {
 template <int NT>
 static cudaError_t launch_nt(const SkinnyParams &p, int grid, size_t smem, cudaStream_t st) {
     void (*kernel)(SkinnyParams) = p.norm_w != nullptr ? skinny_linear_kernel<NT, SK_NORM> : skinny_linear_kernel<NT, SK_PLAIN>;
-    static bool ready[2] = {false, false};
-    const int which = p.norm_w != nullptr ? SK_NORM : SK_PLAIN;
-    if (!ready[which]) {
-        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared);
-        if (e != cudaSuccess) return e;
-        ready[which] = true;
-    }
+    static PerDevice<bool> ready[2];
+    const cudaError_t e = once_per_device(ready[p.norm_w != nullptr ? SK_NORM : SK_PLAIN], [&] {
+        const cudaError_t e1 = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
+        if (e1 != cudaSuccess) return e1;
+        return cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared);
+    });
+    if (e != cudaSuccess) return e;
     return launch_chained(kernel, dim3(grid), dim3(kThreadsSk), smem, st, p);
 }
 

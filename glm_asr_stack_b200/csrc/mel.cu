@@ -228,18 +228,17 @@ __global__ void mel_normalize_kernel(const float *__restrict__ logmel, const flo
         if (f0 + tx < n_frames) o[(size_t)m * n_frames + f0 + tx] = __float2bfloat16(tile[tx][m]);
 }
 
-static int g_mel_smem_ready = 0;
+static PerDevice<bool> g_mel_smem_ready;
 
 // d_num_samples: device array [num_windows].  Returns false on a bad argument.
 bool launch_mel_batched(const float *pcm, long long pcm_stride, const int *d_num_samples, int num_windows, int max_frames,
                         const float *filters_t, __nv_bfloat16 *out, long long out_stride, int time_major, cudaStream_t st) {
     if (num_windows <= 0) return true;
     if (pcm == nullptr || d_num_samples == nullptr || filters_t == nullptr || out == nullptr) return false;
-    if (!g_mel_smem_ready) {
-        if (cudaFuncSetAttribute(mel_power_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(MelSmem)) != cudaSuccess)
-            return false;
-        g_mel_smem_ready = 1;
-    }
+    const cudaError_t ready = once_per_device(g_mel_smem_ready, [] {
+        return cudaFuncSetAttribute(mel_power_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(MelSmem));
+    });
+    if (ready != cudaSuccess) return false;
     float *logmel = (float *)workspace_slot(WS_MEL_LOG, (size_t)num_windows * kMaxFrames * kMels * sizeof(float));
     float *win_max = (float *)workspace_slot(WS_MEL_MAX, (size_t)num_windows * sizeof(float));
     if (cudaMemsetAsync(win_max, 0xFF, (size_t)num_windows * sizeof(float), st) != cudaSuccess) return false;

@@ -307,15 +307,13 @@ bool launch_paged_decode_attention_mma(__nv_bfloat16 *out, int ldo, const __nv_b
     if (q_packed != nullptr && (q_sf == nullptr || !(q_input_scale > 0.0f) || (((uintptr_t)q_packed) & 7) != 0)) return false;
     const int q_sf_chunks = num_q_heads * head_dim / 64;
     const float q_inv_in = q_packed != nullptr ? 1.0f / q_input_scale : 0.0f;
-    static bool configured = false;
-    if (!configured) {
-        if (cudaFuncSetAttribute(paged_decode_attention_mma_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 kAttnSmem) != cudaSuccess ||
-            cudaFuncSetAttribute(paged_decode_attention_mma_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 kAttnSmem) != cudaSuccess)
-            return false;
-        configured = true;
-    }
+    static PerDevice<bool> configured;
+    const cudaError_t ready = once_per_device(configured, [] {
+        const cudaError_t e = cudaFuncSetAttribute(paged_decode_attention_mma_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kAttnSmem);
+        if (e != cudaSuccess) return e;
+        return cudaFuncSetAttribute(paged_decode_attention_mma_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kAttnSmem);
+    });
+    if (ready != cudaSuccess) return false;
     GLMASR_PREFER_MAX_SMEM(paged_decode_attention_mma_kernel<true>);
     GLMASR_PREFER_MAX_SMEM(paged_decode_attention_mma_kernel<false>);
     const float scale = 1.0f / sqrtf((float)head_dim);
@@ -614,12 +612,9 @@ bool launch_paged_decode_split(__nv_bfloat16 *out, int ldo, const __nv_bfloat16 
     const int tiles = (max_len + kTile - 1) / kTile;
     int splits = 1;
     while (q_packed == nullptr && splits < 8 && num_seqs * num_kv_heads * splits * 2 <= 444 && tiles >= splits * 4) splits *= 2;
-    static bool configured = false;
-    if (!configured) {
-        if (cudaFuncSetAttribute(paged_decode_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kAttnSmem) != cudaSuccess)
-            return false;
-        configured = true;
-    }
+    static PerDevice<bool> configured;
+    if (once_per_device(configured, [] { return cudaFuncSetAttribute(paged_decode_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kAttnSmem); }) != cudaSuccess)
+        return false;
     GLMASR_PREFER_MAX_SMEM(paged_decode_split_kernel);
     cudaLaunchConfig_t cfg;
     memset(&cfg, 0, sizeof(cfg));

@@ -261,13 +261,11 @@ bool launch_prefill_attention(__nv_bfloat16 *out, int ldo, const __nv_bfloat16 *
     if ((ldq % 2) != 0 || (ldo % 2) != 0 || (ldk % 8) != 0 || (ldv % 8) != 0) return false;
     if ((((uintptr_t)k | (uintptr_t)v) & 15) != 0 || (((uintptr_t)q | (uintptr_t)out) & 3) != 0) return false;
     if (num_seqs <= 0 || max_seq_len <= 0) return true;
-    static bool configured = false;
-    if (!configured) {
-        if (cudaFuncSetAttribute(prefill_attention_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, AttnCfg<128>::kSmem) !=
-            cudaSuccess)
-            return false;
-        configured = true;
-    }
+    static PerDevice<bool> configured;
+    const cudaError_t ready = once_per_device(configured, [] {
+        return cudaFuncSetAttribute(prefill_attention_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, AttnCfg<128>::kSmem);
+    });
+    if (ready != cudaSuccess) return false;
     const dim3 grid((max_seq_len + kQTile - 1) / kQTile, num_q_heads, num_seqs);
     const float scale = 1.0f / sqrtf((float)head_dim);
     if (head_dim == 128) {

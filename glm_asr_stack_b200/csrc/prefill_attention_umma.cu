@@ -526,14 +526,14 @@ bool launch_prefill_attention_umma(__nv_bfloat16 *out, int ldo, const __nv_bfloa
     if (head_dim == 64)
         return launch_attention64_umma(out, ldo, q, ldq, k, ldk, v, ldv, seq_offsets, seq_lens, num_seqs, max_seq_len, total_tokens,
                                        num_q_heads, num_kv_heads, causal, st);
-    static bool configured = false;
-    if (!configured) {
-        if (cudaFuncSetAttribute(prefill_attention_umma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, G::SMEM_BYTES) != cudaSuccess)
-            return false;
-        cudaFuncSetAttribute(prefill_attention_umma_kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
-                             (int)cudaSharedmemCarveoutMaxShared);
-        configured = true;
-    }
+    static PerDevice<bool> configured;
+    const cudaError_t ready = once_per_device(configured, [] {
+        const cudaError_t e = cudaFuncSetAttribute(prefill_attention_umma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, G::SMEM_BYTES);
+        if (e != cudaSuccess) return e;
+        return cudaFuncSetAttribute(prefill_attention_umma_kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                    (int)cudaSharedmemCarveoutMaxShared);
+    });
+    if (ready != cudaSuccess) return false;
     AttnParams p;
     memset(&p, 0, sizeof(p));
     if (!make_bf16_tmap_sw128(&p.tm_q, q, (uint64_t)num_q_heads * HD, (uint64_t)total_tokens, (uint64_t)ldq * 2, 64, 128)) return false;

@@ -11,6 +11,8 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include "per_device.h"
+
 namespace glmasr {
 
 cudaStream_t current_stream();
