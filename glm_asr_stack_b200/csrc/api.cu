@@ -577,6 +577,7 @@ static bool skinny_eligible(const FusedArgs &a) {
     return skinny_covers(route_rows(a), a.K, rows, a.num_w, a.epi);
 }
 
+// 1 (nothing launched) when the runtime refuses the launch: the caller goes on to the other kernels.
 static int run_skinny(const FusedArgs &a, const __nv_bfloat16 *norm_w = nullptr, float eps = 0.0f) {
     SkinnyParams p;
     memset(&p, 0, sizeof(p));
@@ -604,7 +605,10 @@ static int run_skinny(const FusedArgs &a, const __nv_bfloat16 *norm_w = nullptr,
     p.status = device_status_word();
     profile_bracket_begin(2.0 * a.M * n_rows * a.K, 0.5625 * n_rows * a.K + 2.0 * a.M * (a.K + total_out_cols(a)));
     p.late_trigger = late_trigger_asked() ? 1 : 0;
-    if (launch_skinny_linear(p, num_sms(), g_stream) != cudaSuccess) return -1;
+    if (launch_skinny_linear(p, num_sms(), g_stream) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return 1;
+    }
     note_late_trigger(p.late_trigger != 0);
     profile_bracket_end();
     ++g_launches;
@@ -627,7 +631,7 @@ int fp4_linear_w4a16_normed(uint16_t *out, int ldo, const uint16_t *x, const uin
     a.M = M;
     a.K = K;
     if (!tensor_core_eligible(a) || !aligned16(norm_w) || !skinny_eligible(a)) return -1;
-    return run_skinny(a, (const __nv_bfloat16 *)norm_w, eps);
+    return run_skinny(a, (const __nv_bfloat16 *)norm_w, eps) == 0 ? 0 : -1;
 }
 
 // GLMASR_CLUSTER_ROWS=n: most rows that the cluster split-K bf16 GEMM takes (comparison runs; 0: never)
@@ -642,7 +646,8 @@ static int cluster_gemm_rows() {
     return v;
 }
 
-// bf16 GEMM on the cluster split-K kernel; 1 (nothing launched) when the other kernels are expected to be faster.
+// bf16 GEMM on the cluster split-K kernel; 1 (nothing launched) when the other kernels are expected to be faster or the launch
+// is refused.
 static int run_cluster(const FusedArgs &a) {
     ClusterGemmParams p;
     memset(&p, 0, sizeof(p));
@@ -681,7 +686,10 @@ static int run_cluster(const FusedArgs &a) {
     profile_bracket_begin(2.0 * a.M * n_rows * a.K, 2.0 * n_rows * a.K + 2.0 * a.M * (a.K + total_out_cols(a)) +
                                                         (a.epi == EPI_RESIDUAL ? 2.0 * a.M * total_out_cols(a) : 0.0));
     p.late_trigger = late_trigger_asked() ? 1 : 0;
-    if (launch_cluster_gemm(p, g_stream) != cudaSuccess) return -1;
+    if (launch_cluster_gemm(p, g_stream) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return 1;
+    }
     note_late_trigger(p.late_trigger != 0);
     profile_bracket_end();
     ++g_launches;
@@ -705,7 +713,10 @@ static int run_fused(const FusedArgs &a) {
     }
 
     // W4A16 with a handful of rows: the few-row kernel reads the packed weights as they are.
-    if (skinny_eligible(a)) return run_skinny(a);
+    if (skinny_eligible(a)) {
+        const int rc = run_skinny(a);
+        if (rc <= 0) return rc;
+    }
 
     // W4A16 on resident bf16 copies of the weights (made on first use, within the budget): the bf16 GEMM streams
     // them at the rate of the memory system, where the in-kernel dequant of a decode-sized call is a chain of
