@@ -141,6 +141,10 @@ __global__ void __launch_bounds__(kCgThreads, 2) cluster_gemm_kernel(const __gri
     }
     pdl_wait();                         // residual, bias and out belong to the preceding kernels until here
     __syncthreads();                    // the ring is dead: every load of it has been consumed by a completed MMA
+    if (*abort_word != 0) {             // ... unless a wait ran out: let loads and MMAs in flight end before their memory is reused
+        for (int i = 0; i < 64; ++i) __nanosleep(1000);
+        __syncthreads();
+    }
     tc_fence_after();
     // accumulator -> shared memory as [token][128 weight rows] fp32 (a warp stores 32 consecutive rows of a token)
     float *part = reinterpret_cast<float *>(cg_raw + (ring - raw));

@@ -257,7 +257,10 @@ __global__ void __launch_bounds__(kThreadsSk, 2) skinny_linear_kernel(const __gr
                 }
             }
             __syncthreads();
-            if (*abort_word != 0) return;
+            if (*abort_word != 0) {
+                for (int i = 0; i < 64; ++i) __nanosleep(1000);     // let copies in flight land
+                return;
+            }
             // sum over the warps, epilogue: a thread per (unit, token, row), rows fastest
             const int units = (min(tiles, t0 + R) - t0) / mt;
             for (int i = threadIdx.x; i < units * 16 * p.M; i += kThreadsSk) {
