@@ -56,18 +56,19 @@ static size_t ln_smem_bytes(int dim) { return (size_t)dim * 4 + (size_t)kLnRows 
 
 __global__ void __launch_bounds__(kLnWarps * 32, 8) layernorm_kernel(__nv_bfloat16 *out, const __nv_bfloat16 *x,
                                                                   const __nv_bfloat16 *weight, const __nv_bfloat16 *bias,
-                                                                  float eps, int rows, int dim) {
+                                                                  float eps, int rows, int dim, int early_weights) {
     extern __shared__ __align__(16) uint8_t ln_smem[];
     uint4 *w_s = reinterpret_cast<uint4 *>(ln_smem), *b_s = w_s + (dim >> 3);
     pdl_launch_dependents();
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, vecs = dim >> 3;
     const int row0 = blockIdx.x * kLnRows + wib * 2;
     uint8_t *rows_s = ln_smem + (size_t)dim * 4 + (size_t)wib * 2 * (dim * 2 + 64);     // 64 bytes apart: other banks
+    if (!early_weights) pdl_wait();
     for (int i = threadIdx.x; i < vecs; i += kLnWarps * 32) {
         w_s[i] = reinterpret_cast<const uint4 *>(weight)[i];
         b_s[i] = bias != nullptr ? reinterpret_cast<const uint4 *>(bias)[i] : make_uint4(0u, 0u, 0u, 0u);
     }
-    pdl_wait();
+    if (early_weights) pdl_wait();
 #pragma unroll
     for (int r = 0; r < 2; ++r)
         if (row0 + r < rows) {
@@ -169,7 +170,7 @@ void launch_layernorm(__nv_bfloat16 *out, const __nv_bfloat16 *x, const __nv_bfl
     const bool vec = (dim % 8) == 0 && (((uintptr_t)out | (uintptr_t)x | (uintptr_t)weight | (uintptr_t)bias) & 15) == 0;
     if (dim <= 1280 && vec)          // eight rows fit 48 KB of shared memory (the encoder's 1280)
         launch_chained(layernorm_kernel, dim3((rows + kLnRows - 1) / kLnRows), dim3(kLnWarps * 32), ln_smem_bytes(dim), st, out, x,
-                       weight, bias, eps, rows, dim);
+                       weight, bias, eps, rows, dim, weights_settled() ? 1 : 0);
     else
         launch_chained(layernorm_generic_kernel, dim3((rows + 7) / 8), dim3(256), (size_t)0, st, out, x, weight, bias, eps, rows, dim);
     note_launches(1);
@@ -545,9 +546,10 @@ static void encoder_layers(const glmasr_WeightStore *ws, const glmasr_ModelConfi
     uint16_t *ffn = (uint16_t *)workspace_slot(WS_E_FFN, (size_t)M * F * 2);
     int *row_pos = (int *)workspace_slot(WS_E_POS, (size_t)M * sizeof(int));
     {
-        PlainLaunch plain(true);        // the GEMMs behind it fetch their weights early
+        PlainLaunch plain(true);        // the GEMMs and norms behind it fetch their weights early
         launch_chained(fill_row_positions_kernel, dim3(8, num_seqs), dim3(256), (size_t)0, st, row_pos, d_offsets, d_lens, num_seqs);
     }
+    SettledWeights settled(true);
     note_launches(1);
     for (int l = 0; l < L; ++l) {
         const EncLayerRef &W = R.layers[l];

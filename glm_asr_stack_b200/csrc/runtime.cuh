@@ -65,7 +65,7 @@ bool pdl_enabled();
 // completed before the kernel in FRONT of it started.  An ordinary launch (no attribute) starts when everything before
 // it has completed, so one such launch between the writer and the chain settles that for all kernels behind it.
 // PlainLaunch makes the launches of its scope ordinary ones; SettledWeights marks the scope of a driver whose first
-// launch was ordinary, in which the caller's packed weights may be fetched early.
+// launch was ordinary, in which the caller's weights may be fetched early; outside of it a kernel waits first.
 struct PlainLaunch {
     explicit PlainLaunch(bool on);
     ~PlainLaunch();

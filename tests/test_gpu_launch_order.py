@@ -67,3 +67,15 @@ def test_bf16_weight_computed_in_front_of_its_linear(ops, M):
     one = torch.ones(512, dtype=torch.bfloat16, device="cuda")
     w = torch.empty((1024, 512), dtype=torch.bfloat16, device="cuda")
     check(ops, lambda i: ops.rmsnorm(src[i], one, out=w), lambda: ops.bf16_linear(x, w))
+
+
+@pytest.mark.parametrize("rows", [1, 200, 4000])
+def test_layernorm_weights_computed_in_front_of_it(ops, rows):
+    dim = 1280
+    gen = torch.Generator(device="cuda").manual_seed(rows)
+    x = torch.randn((rows, dim), generator=gen, device="cuda").to(torch.bfloat16)
+    src = [torch.randn((2048, dim), generator=gen, device="cuda").to(torch.bfloat16) for _ in range(7)]
+    one = torch.ones(dim, dtype=torch.bfloat16, device="cuda")
+    params = torch.empty((2048, dim), dtype=torch.bfloat16, device="cuda")
+    # the last rows of a norm over many: what its last CTAs write
+    check(ops, lambda i: ops.rmsnorm(src[i], one, out=params), lambda: ops.layernorm(x, params[2046], params[2047]))
