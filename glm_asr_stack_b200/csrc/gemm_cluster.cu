@@ -141,10 +141,6 @@ __global__ void __launch_bounds__(kCgThreads, 2) cluster_gemm_kernel(const __gri
     }
     pdl_wait();                         // residual, bias and out belong to the preceding kernels until here
     __syncthreads();                    // the ring is dead: every load of it has been consumed by a completed MMA
-    if (*abort_word != 0) {             // ... unless a wait ran out: let loads and MMAs in flight end before their memory is reused
-        for (int i = 0; i < 64; ++i) __nanosleep(1000);
-        __syncthreads();
-    }
     tc_fence_after();
     // accumulator -> shared memory as [token][128 weight rows] fp32 (a warp stores 32 consecutive rows of a token)
     float *part = reinterpret_cast<float *>(cg_raw + (ring - raw));
@@ -267,8 +263,14 @@ __global__ void __launch_bounds__(kCgThreads, 2) cluster_gemm_kernel(const __gri
     }
     if (p.splits > 1) cluster_sync_all();       // nobody leaves while its shares are being read
     else __syncthreads();
-    if (threadIdx.x == 0 && *abort_word != 0 && p.status != nullptr) atomicCAS(p.status, 0, *abort_word);
-    if (warp == 1) tmem_dealloc(tmem, cols);
+    if (warp <= 1) {
+        if (*abort_word != 0) {         // a wait ran out: let loads and MMAs in flight end before their memory is given up
+            for (int i = 0; i < 64; ++i) __nanosleep(1000);
+            if (threadIdx.x == 0 && p.status != nullptr) atomicCAS(p.status, 0, *abort_word);
+        }
+        __syncwarp();
+        if (warp == 1) tmem_dealloc(tmem, cols);
+    }
 }
 
 static size_t cg_smem_bytes(int n_tok, int stages) {
@@ -313,15 +315,12 @@ static cudaError_t cg_ready() {
 
 // Clusters of `splits` CTAs that the device holds at once at this shared-memory size (graphics processing clusters have
 // 16 to 20 SMs here, so it is less than 148 * 2 / splits), 0 when it holds none; asked once per pair and device.
-static int cg_max_clusters(int splits, size_t smem) {
-    struct Known {
-        int n[9][16];               // 0: not asked yet, -1: none
-    };
-    static PerDevice<Known> known;
-    Known *k = known.here();
-    if (k == nullptr) return 0;
+struct ClustersKnown {
+    int n[9][16];                   // 0: not asked yet, -1: none
+};
+static int cg_max_clusters(ClustersKnown &known, int splits, size_t smem) {
     const int slot = (int)(smem >> 14) & 15;
-    int &v = k->n[splits][slot];
+    int &v = known.n[splits][slot];
     if (v == 0) {
         cudaLaunchConfig_t cfg;
         cudaLaunchAttribute attr[2];
@@ -343,6 +342,9 @@ static int cg_max_clusters(int splits, size_t smem) {
 double choose_cluster_gemm(ClusterGemmParams &p, int w_tiles) {
     if (p.M < 1 || p.M > kClusterMaxRows || p.k_blocks < 1 || w_tiles < 1) return 0.0;
     if (cg_ready() != cudaSuccess) return 0.0;
+    static PerDevice<ClustersKnown> per_device;
+    ClustersKnown *known = per_device.here();
+    if (known == nullptr) return 0.0;
     p.w_tiles = w_tiles;
     double best = 1e30;
     for (int tt = (p.M + 255) / 256; tt <= (p.M + 63) / 64; ++tt) {
@@ -355,7 +357,7 @@ double choose_cluster_gemm(ClusterGemmParams &p, int w_tiles) {
         const size_t smem = cg_smem_bytes(n_tok, stages);
         for (int c = 1; c <= 8 && (c == 1 || c * 2 <= p.k_blocks); ++c) {
             const int clusters = w_tiles * tt;
-            const int room = cg_max_clusters(c, smem);
+            const int room = cg_max_clusters(*known, c, smem);
             if (room == 0) continue;
             const double waves = (clusters + room - 1) / room;
             const double share = clusters * c > 148 && smem <= 113 * 1024 ? 2.0 : 1.0;
