@@ -469,7 +469,9 @@ static int total_out_cols(const FusedArgs &a) {
 }
 
 // SIMT route: same results, any shape.
+static int g_last_route = GLMASR_ROUTE_NONE;
 static int run_simt(const FusedArgs &a) {
+    g_last_route = GLMASR_ROUTE_SIMT;
     const uint8_t *xq = nullptr, *xs = nullptr;
     const __nv_bfloat16 *x = a.x;
     int ldx = a.ldx;
@@ -574,7 +576,9 @@ static bool skinny_eligible(const FusedArgs &a) {
     if (a.mode != GEMM_W4A16 || a.pre != nullptr || a.q_out != nullptr) return false;
     int rows[kMaxSegments];
     for (int i = 0; i < a.num_w; ++i) rows[i] = a.w[i].N;
-    return skinny_covers(route_rows(a), a.K, rows, a.num_w, a.epi);
+    // without resident copies what follows dequantises inside the GEMM, the slowest of the three
+    return skinny_covers(route_rows(a), a.K, rows, a.num_w, a.epi) &&
+           (resident_budget_bytes() == 0 || skinny_pays(route_rows(a), a.K, rows, a.num_w, a.epi, num_sms()));
 }
 
 // 1 (nothing launched) when the runtime refuses the launch: the caller goes on to the other kernels.
@@ -605,10 +609,12 @@ static int run_skinny(const FusedArgs &a, const __nv_bfloat16 *norm_w = nullptr,
     p.status = device_status_word();
     profile_bracket_begin(2.0 * a.M * n_rows * a.K, 0.5625 * n_rows * a.K + 2.0 * a.M * (a.K + total_out_cols(a)));
     p.late_trigger = late_trigger_asked() ? 1 : 0;
-    if (launch_skinny_linear(p, num_sms(), g_stream) != cudaSuccess) {
+    int rounds = 0;
+    if (launch_skinny_linear(p, num_sms(), g_stream, &rounds) != cudaSuccess) {
         (void)cudaGetLastError();
         return 1;
     }
+    g_last_route = GLMASR_ROUTE_FEW_ROWS | rounds << 8;
     note_late_trigger(p.late_trigger != 0);
     profile_bracket_end();
     ++g_launches;
@@ -690,6 +696,7 @@ static int run_cluster(const FusedArgs &a) {
         (void)cudaGetLastError();
         return 1;
     }
+    g_last_route = GLMASR_ROUTE_CLUSTER | p.splits << 8;
     note_late_trigger(p.late_trigger != 0);
     profile_bracket_end();
     ++g_launches;
@@ -937,6 +944,7 @@ static int run_fused(const FusedArgs &a) {
             } else if ((pair_bf16 ? launch_umma_gemm_pair_bf16(p, pairs, g_stream) : launch_umma_gemm_pair(p, pairs, g_stream)) != cudaSuccess) {
                 return -1;
             }
+            g_last_route = GLMASR_ROUTE_PAIR;
             ++g_launches;
             if (g_profile) {
                 cudaEventRecord(tl.stop, g_stream);
@@ -1005,6 +1013,7 @@ static int run_fused(const FusedArgs &a) {
         cudaEventRecord(tl.start, g_stream);
     }
     if (launch_umma_gemm(a.mode, nb, p, ctas, g_stream) != cudaSuccess) return -1;
+    g_last_route = GLMASR_ROUTE_TILE;
     ++g_launches;
     if (g_profile) {
         cudaEventRecord(tl.stop, g_stream);
@@ -1640,6 +1649,8 @@ extern "C" int glmasr_fp4_status(void) {
     }
     return code;
 }
+
+extern "C" int glmasr_last_gemm_route(void) { return g_last_route; }
 
 extern "C" long long glmasr_launch_count(void) { return g_launches; }
 

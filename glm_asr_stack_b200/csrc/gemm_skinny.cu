@@ -315,6 +315,27 @@ bool skinny_covers(int M, int K, const int *seg_rows, int num_segs, int epi) {
     return true;
 }
 
+// The other route reads bf16 copies, 3.6 times the bytes; this one pays for dequantising and, per CTA, for the rows' operand in
+// every pass.  Both sides in us, weights not in L2, this kernel / the other:
+//   * weights of a CTA all requested up front (they fit the slots), K >= 1536: 2048 x 6144 8.9 / 24.8 (1 row), 12.4 / 24.8 (16);
+//     12288 x 2048 9.3 / 20.6, 15.2 / 19.8; 8192 x 4096 11.9 / 30, 14.8 / 19.6; 4096 x 8192 13.3 / 41, 16.5 / 32: always;
+//   * taller ones go through the ring.  Below 128 KB of rows the other route is slow as well: 24576 x 2048 16.4 / 32 (1), 24.5 / 30
+//     (16); 59264 x 2048 34.6 / 58, 50.9 / 53 (12) but 55 / 52 (16); 24576 x 6144 59 / 85, 81 / 88 (9).  From 128 KB of rows on it
+//     is not: 16384 x 8192 58 / 49 (8), 66 / 49 (16); 8192 x 6144 32 / 27 (12); 12288 x 4096 26 / 23 (16);
+//   * K below 1536 leaves warps without a chunk and units too short: 9472 x 1024 5.4 / 9.6 (1), 7.3 / 9.3 (16), 16384 x 1024 10.8 / 11.9
+//     (8), 14.6 / 11.6 (16); 9472 x 512 5.5 / 6.3 (8), 7.0 / 6.3 (16), 16384 x 512 8.6 / 7.7 (8); 16384 x 256 7.0 / 5.9 (1).
+bool skinny_pays(int M, int K, const int *seg_rows, int num_segs, int epi, int num_sms) {
+    const int mt = epi == EPI_SILU_GATE ? 2 : 1;
+    int rows = 0;
+    for (int i = 0; i < (mt == 2 ? 1 : num_segs); ++i) rows += seg_rows[i];
+    const int tiles = (rows / 16 + num_sms - 1) / num_sms * mt;         // 16-row tiles of a CTA
+    if (K < 512) return M <= 8 && tiles <= 1;
+    if (K < 1024) return tiles <= (M <= 8 ? 4 : 1);
+    if (K < 1536) return M <= 8 || tiles <= 4;
+    if (tiles * sk_slot_bytes(K) <= kSmemWeights) return true;
+    return M * K < 65536 && !(M > 12 && tiles > 20);
+}
+
 template <int NT>
 static cudaError_t launch_nt(const SkinnyParams &p, int grid, size_t smem, cudaStream_t st) {
     void (*kernel)(SkinnyParams) = p.norm_w != nullptr ? skinny_linear_kernel<NT, SK_NORM> : skinny_linear_kernel<NT, SK_PLAIN>;
@@ -328,7 +349,7 @@ static cudaError_t launch_nt(const SkinnyParams &p, int grid, size_t smem, cudaS
     return launch_chained(kernel, dim3(grid), dim3(kThreadsSk), smem, st, p);
 }
 
-cudaError_t launch_skinny_linear(SkinnyParams p, int num_sms, cudaStream_t st) {
+cudaError_t launch_skinny_linear(SkinnyParams p, int num_sms, cudaStream_t st, int *rounds) {
     if (!skinny_covers(p.M, p.K, p.seg_rows, p.num_segs, p.epi)) return cudaErrorInvalidValue;
     const int mt = p.epi == EPI_SILU_GATE ? 2 : 1;
     int rows = 0;
@@ -348,6 +369,7 @@ cudaError_t launch_skinny_linear(SkinnyParams p, int num_sms, cudaStream_t st) {
         if (p.units_per_group < 1) p.groups = 1, p.units_per_group = 1;
     }
     const int grid = (p.units + p.units_per_cta - 1) / p.units_per_cta;
+    *rounds = (p.units_per_cta + p.units_per_group - 1) / p.units_per_group;
     p.pass_tiles = sk_tiles_per_pass(nt) < p.units_per_group * mt ? sk_tiles_per_pass(nt) : p.units_per_group * mt;
     const size_t smem = kSmemHeader + (size_t)p.groups * p.units_per_group * unit_bytes +
                         (size_t)kWarpsSk * p.pass_tiles * 16 * nt * 8 * sizeof(float);

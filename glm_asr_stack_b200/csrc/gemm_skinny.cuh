@@ -33,6 +33,9 @@ struct SkinnyParams {
 
 // cudaErrorInvalidValue when the shape is not covered (nothing launched).
 bool skinny_covers(int M, int K, const int *seg_rows, int num_segs, int epi);
-cudaError_t launch_skinny_linear(SkinnyParams p, int num_sms, cudaStream_t st);
+// Whether the kernel is the faster route for a shape that it covers (the other one: bf16 copies of the weights).
+bool skinny_pays(int M, int K, const int *seg_rows, int num_segs, int epi, int num_sms);
+// *rounds: rounds in which a CTA reads its weights.
+cudaError_t launch_skinny_linear(SkinnyParams p, int num_sms, cudaStream_t st, int *rounds);
 
 }  // namespace glmasr

@@ -540,6 +540,15 @@ def status() -> int:
     return _lib.load().glmasr_fp4_status()
 
 
+ROUTES = ("none", "simt", "tile", "pair", "few_rows", "cluster")
+
+
+def last_gemm_route():
+    """(name of the kernel that served the last linear, its CTAs per share of K or rounds): glmasr_last_gemm_route."""
+    r = _lib.load().glmasr_last_gemm_route()
+    return ROUTES[r & 255], r >> 8
+
+
 def launch_count() -> int:
     return int(_lib.load().glmasr_launch_count())
 

@@ -373,6 +373,16 @@ int glmasr_nvfp4_linear_noalloc(uint16_t *out, const uint16_t *x, const uint8_t 
  * (0 = none; 1..6 = a bounded wait inside a kernel ran out, 7 = a layout a kernel cannot work with),
  * then clear it. */
 int glmasr_fp4_status(void);
+/* Which kernel served the last linear of this library (any of the FP4 / bf16 linears; a layer or a driver: its last GEMM):
+ * bits 0-7 one of GLMASR_ROUTE_*, bits 8 and up the CTAs that share K (GLMASR_ROUTE_CLUSTER) or the rounds in which a CTA
+ * reads its weights (GLMASR_ROUTE_FEW_ROWS).  For tests and profiles; no reference counterpart. */
+#define GLMASR_ROUTE_NONE     0
+#define GLMASR_ROUTE_SIMT     1   /* any shape and alignment */
+#define GLMASR_ROUTE_TILE     2   /* tcgen05, a CTA per 128-row tile */
+#define GLMASR_ROUTE_PAIR     3   /* tcgen05, a CTA pair per 256-row tile */
+#define GLMASR_ROUTE_FEW_ROWS 4   /* W4A16 on the packed weights, up to 16 rows */
+#define GLMASR_ROUTE_CLUSTER  5   /* tcgen05, K cut over a cluster, up to 512 rows */
+int glmasr_last_gemm_route(void);
 /* Number of kernels this library has launched since load (for launch accounting). */
 long long glmasr_launch_count(void);
 /* Per-launch timing of the tensor-core GEMM kernel with CUDA events recorded on the launching

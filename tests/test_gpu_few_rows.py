@@ -1,4 +1,4 @@
-"""The few-row FP4 linear (1 to 16 rows of W4A16, 1 to 8 of a single W4A4 linear) at the edges of its token tiles (8, 16),
+"""The few-row FP4 linear (1 to 16 rows of W4A16) at the edges of its token tiles (8, 16),
 of its 16-row units and of its chunks of K, and the first sizes of the bf16 route behind it, against the float32 oracles.  Tolerance: one bf16 rounding of the result
 (2^-9) and the order of a float32 sum of at most 8192 exact products, the bar every other route is held to."""
 import numpy as np
@@ -82,3 +82,47 @@ def test_cluster_split_k(ops, M, N, K):
     want = torch.nn.functional.gelu(want, approximate="tanh")
     got = ops.bf16_linear_gelu(x, w, b).double()
     assert float((got - want).norm() / want.norm()) <= REL_TOL_TIGHT
+
+
+def rand_fp4(ops, N, K, seed):
+    """A weight of any size quickly: random codes, scales around one; with it its values in float64."""
+    gen = torch.Generator(device="cuda").manual_seed(seed)
+    packed = torch.randint(0, 256, (N, K // 2), generator=gen, dtype=torch.uint8, device="cuda")
+    scales = torch.randint(48, 64, (N, K // 16), generator=gen, dtype=torch.uint8, device="cuda")
+    lut = torch.tensor([0, .5, 1, 1.5, 2, 3, 4, 6, 0, -.5, -1, -1.5, -2, -3, -4, -6], dtype=torch.float64, device="cuda")
+    v = torch.stack([lut[(packed & 15).long()], lut[(packed >> 4).long()]], -1).view(N, K // 16, 16)
+    return ops.Fp4Tensor(packed, scales, 0.25), (v * scales.view(torch.float8_e4m3fn).double()[..., None] * 0.25).view(N, K)
+
+
+@pytest.mark.parametrize("N,K,rounds", [(4752, 8192, 3), (20000, 2048, 2), (16 * 1333, 3072, 4)])
+@pytest.mark.parametrize("M", [1, 7, 9, 15])
+def test_weights_read_in_rounds(ops, N, K, rounds, M):
+    """Weights too tall for one round: slots refilled, barrier phases, row sums kept, a last CTA with fewer units.  The shapes
+    that take the other route by their size (128 KB of rows and more) are held to the same bar."""
+    w, dense = rand_fp4(ops, N, K, N + M)
+    x = to_dev_bf16(o.seeded_activation(M, K, M))
+    got = ops.fp4_linear(x, w.w_packed, w.w_scales, w.w_global_scale)
+    route = ops.last_gemm_route()
+    if M * K < 65536:
+        assert route[0] == "few_rows" and route[1] >= rounds, route
+    else:
+        assert route[0] != "few_rows", route
+    want = x.double() @ dense.T
+    assert float((got.double() - want).norm() / want.norm()) <= REL_TOL_TIGHT
+    gate = ops.fp4_linear_fused(ops.MODE_W4A16, x, [w, w], epilogue=ops.EPI_SILU_GATE)
+    want = want.to(torch.bfloat16).double()
+    want = want * torch.sigmoid(want) * want
+    assert float((gate.double() - want).norm() / want.norm()) <= REL_TOL_VS_ORACLE
+
+
+@pytest.mark.parametrize("M,N,K,few", [(8, 2048, 6144, True), (16, 12288, 2048, True), (16, 4096, 8192, True), (8, 59264, 2048, True),
+                                       (16, 59264, 2048, False), (8, 16384, 8192, False), (12, 8192, 6144, False), (16, 16384, 1024, False),
+                                       (8, 16384, 512, False), (16, 4096, 256, False), (17, 2048, 2048, False)])
+def test_route_is_the_faster_one(ops, M, N, K, few):
+    """Sizes on both sides of the rule, each measured (skinny_pays); the result is the same up to the sum's order either way."""
+    w, dense = rand_fp4(ops, N, K, 5)
+    x = to_dev_bf16(o.seeded_activation(M, K, M))
+    got = ops.fp4_linear(x, w.w_packed, w.w_scales, w.w_global_scale)
+    assert (ops.last_gemm_route()[0] == "few_rows") == few
+    want = x.double() @ dense.T
+    assert float((got.double() - want).norm() / want.norm()) <= REL_TOL_TIGHT
