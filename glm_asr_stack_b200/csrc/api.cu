@@ -670,12 +670,15 @@ static int run_cluster(const FusedArgs &a) {
         if (i == 0 || !silu) tiles += p.seg_tiles[i];
         n_rows += a.n_bf16[i];
     }
-    // the single-CTA kernel, in a chain of launches: 5.5 us and 0.2 us per 64-wide k block of a 128 x 128 tile, one tile per
-    // SM and round; gate and up are one tile of twice that (measured: 185 x 1280 x 1280 11 us, 185 x 3840 x 1280 9.4,
-    // 173 x 2048 x 6144 24.7, gate|up of 19 and of 173 rows with K = 2048 19.5; this kernel: 8.9, -, 17.8, 12.8 for 19 rows)
-    const double cluster_ns = choose_cluster_gemm(p, tiles);
+    // The single-CTA kernel, fitted to the same launches (5.5 %): 3.4 us, 0.225 us per 64-wide k block of a 128 x 128 tile, one tile
+    // per SM and round (gate and up: one tile of 2.1 times that), up to 1 us for the rows of the epilogue, 1.35 us for a residual.
+    // Within 3 % of each other the single-CTA kernel keeps the shape.  Measured, this kernel / the single-CTA one: 1280 x 1280
+    // 5.7 / 7.8 us (17 rows), 8.0 / 8.6 (185), 9.4 / 8.5 (257); 2048 x 6144 9.0 / 24.8 (17), 16 / 24.9 (185); 2048 x 2048
+    // 10.5 / 11.4 (173), 14.9 / 11.8 (384); gate|up of K = 2048 13.4 / 19.1 (17), 25 / 19.2 (129).
+    const double cluster_ns = choose_cluster_gemm(p, tiles, num_sms());
+    const double row_ns = 1014.0 * (a.M < 128 ? a.M : 128) / 128 + (a.epi == EPI_RESIDUAL ? 1350.0 : 0.0);
     const int rounds = ((a.M + 127) / 128 * (silu ? (a.n_bf16[0] + 127) / 128 : tiles) + num_sms() - 1) / num_sms();
-    if (cluster_ns == 0.0 || cluster_ns > 5500.0 + (silu ? 400.0 : 200.0) * p.k_blocks * rounds) return 1;
+    if (cluster_ns == 0.0 || cluster_ns > 0.97 * (3380.0 + (silu ? 473.0 : 225.0) * p.k_blocks * rounds + row_ns)) return 1;
     for (int i = 0; i < a.num_w; ++i)
         if (!make_tmap(&p.tm_w[i], a.w_bf16[i], CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)a.K, (uint64_t)a.n_bf16[i],
                        (uint64_t)a.K * 2, 64, silu ? 64 : 128, true))

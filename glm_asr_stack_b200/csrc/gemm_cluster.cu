@@ -339,10 +339,11 @@ static int cg_max_clusters(ClustersKnown &known, int splits, size_t smem) {
     return v > 0 ? v : 0;
 }
 
-// Times in ns, fitted to launches of this kernel on a B200 (19 to 256 rows, K 1280 to 6144; within 15 %): a fixed 3.5 us,
-// then the slower of the operand stream -- an SM takes 118 bytes per ns, shared-memory writes and MMA reads together --
-// and the ring's round trips of 1.3 us, then the reduction.
-double choose_cluster_gemm(ClusterGemmParams &p, int w_tiles) {
+// Times in ns, fitted to 471 launches of this kernel on a B200 (sixteen shapes of K 384 to 6144 and 512 to 8192 columns, 1 to 512
+// rows, chains of launches, weights not in L2; standard deviation 7 %, the short K = 384 up to 26 % too high): a fixed 2.9 us,
+// then the slower of the operand stream -- 190 bytes per ns and SM -- and the ring's round trips of 1.2 us, then the shares'
+// way through distributed shared memory, 2.7 TB/s for the whole chip, or the one accumulator's through the CTA's own.
+double choose_cluster_gemm(ClusterGemmParams &p, int w_tiles, int num_sms) {
     if (p.M < 1 || p.M > kClusterMaxRows || p.k_blocks < 1 || w_tiles < 1) return 0.0;
     if (cg_ready() != cudaSuccess) return 0.0;
     static PerDevice<ClustersKnown> per_device;
@@ -363,11 +364,13 @@ double choose_cluster_gemm(ClusterGemmParams &p, int w_tiles) {
             const int room = cg_max_clusters(*known, c, smem);
             if (room == 0) continue;
             const double waves = (clusters + room - 1) / room;
-            const double share = clusters * c > 148 && smem <= 113 * 1024 ? 2.0 : 1.0;
+            const int per_sm = smem <= 113 * 1024 ? 2 : 1;
+            const double share = clusters * c > num_sms && per_sm == 2 ? 2.0 : 1.0;
+            const int resident = clusters * c < num_sms * per_sm ? clusters * c : num_sms * per_sm;
             const int kb = (p.k_blocks + c - 1) / c;
-            const double stream = 1.25 * kb * stage * share / 118.0, trips = (kb + stages - 1) / stages * 1300.0;
-            double ns = waves * (stream > trips ? stream : trips) + 3500.0;
-            if (c > 1) ns += waves * (1500.0 + n_tok * 512.0 * share / 60.0);
+            const double stream = kb * stage * share / 190.0, trips = (kb + stages - 1) / stages * 1200.0;
+            double ns = waves * (stream > trips ? stream : trips) + 2900.0;
+            ns += waves * (c > 1 ? 1630.0 + n_tok * 512.0 * resident / 2700.0 : n_tok * 22.0 * share);
             if (ns < best) best = ns, p.splits = c, p.n_tok = n_tok, p.token_tiles = tt, p.stages = stages;
         }
     }

@@ -28,7 +28,7 @@ struct alignas(64) ClusterGemmParams {
 
 // Tile shape for `w_tiles` 128-row weight tiles, M tokens and K = 64 * k_blocks.  Returns the time expected of it in ns, 0 when
 // the shape is not covered.
-double choose_cluster_gemm(ClusterGemmParams &p, int w_tiles);
+double choose_cluster_gemm(ClusterGemmParams &p, int w_tiles, int num_sms);
 cudaError_t launch_cluster_gemm(const ClusterGemmParams &p, cudaStream_t st);
 
 }  // namespace glmasr

@@ -126,3 +126,16 @@ def test_route_is_the_faster_one(ops, M, N, K, few):
     assert (ops.last_gemm_route()[0] == "few_rows") == few
     want = x.double() @ dense.T
     assert float((got.double() - want).norm() / want.norm()) <= REL_TOL_TIGHT
+
+
+@pytest.mark.parametrize("M,N,K,cluster", [(17, 2048, 6144, True), (173, 1280, 1280, True), (512, 512, 2048, True), (173, 2048, 2048, True),
+                                           (384, 2048, 2048, False), (320, 1280, 1280, False), (128, 3840, 1280, False), (200, 1280, 384, False),
+                                           (300, 8192, 512, False), (513, 512, 2048, False)])
+def test_cluster_route_is_the_faster_one(ops, M, N, K, cluster):
+    """Sizes on both sides of the estimates, each measured (run_cluster); the result holds either way."""
+    gen = torch.Generator(device="cuda").manual_seed(M + N)
+    x, w = (torch.randn(s, generator=gen, device="cuda").to(torch.bfloat16) for s in ((M, K), (N, K)))
+    got = ops.bf16_linear(x, w).double()
+    assert (ops.last_gemm_route()[0] == "cluster") == cluster
+    want = x.double() @ w.double().T
+    assert float((got - want).norm() / want.norm()) <= REL_TOL_TIGHT
