@@ -383,7 +383,9 @@ bool launch_attention64_umma(__nv_bfloat16 *out, int ldo, const __nv_bfloat16 *q
         if (cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || num_sms <= 0) num_sms = 148;
     }
     const int grid = p.total_items < CTAS_PER_SM * num_sms ? p.total_items : CTAS_PER_SM * num_sms;
-    return launch_chained(attention64_umma_kernel, dim3(grid), dim3(THREADS64), (size_t)SMEM64, st, p) == cudaSuccess;
+    const cudaError_t e = launch_chained(attention64_umma_kernel, dim3(grid), dim3(THREADS64), (size_t)SMEM64, st, p);
+    if (e != cudaSuccess) (void)cudaGetLastError();         // refused: the caller goes on to the warp-level kernel
+    return e == cudaSuccess;
 }
 
 }  // namespace glmasr

@@ -631,10 +631,13 @@ bool launch_paged_decode_split(__nv_bfloat16 *out, int ldo, const __nv_bfloat16 
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = pdl_enabled() ? 2 : 1;
-    return cudaLaunchKernelEx(&cfg, paged_decode_split_kernel, out, ldo, qkv, ld, k_col, v_col, angles, slot_mapping, key_cache,
-                              value_cache, block_tables, seq_lens, num_kv_heads, group, block_size, max_blocks_per_seq,
-                              1.0f / sqrtf((float)head_dim), early_cache && pdl_enabled() ? 1 : 0, q_packed, q_sf,
-                              num_q_heads * head_dim / 64, q_packed != nullptr ? 1.0f / q_input_scale : 0.0f) == cudaSuccess;
+    const cudaError_t launched =
+        cudaLaunchKernelEx(&cfg, paged_decode_split_kernel, out, ldo, qkv, ld, k_col, v_col, angles, slot_mapping, key_cache,
+                           value_cache, block_tables, seq_lens, num_kv_heads, group, block_size, max_blocks_per_seq,
+                           1.0f / sqrtf((float)head_dim), early_cache && pdl_enabled() ? 1 : 0, q_packed, q_sf,
+                           num_q_heads * head_dim / 64, q_packed != nullptr ? 1.0f / q_input_scale : 0.0f);
+    if (launched != cudaSuccess) (void)cudaGetLastError();       // refused: the caller goes on to the separate launches
+    return launched == cudaSuccess;
 }
 
 }  // namespace glmasr
