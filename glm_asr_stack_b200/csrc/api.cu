@@ -188,7 +188,7 @@ enum Slot : int {
     WS_PARTIAL = 30, WS_COUNTERS = 31,   // split-K partial accumulators and per-tile arrival counters   // layer path: quantised SiLU-gate output handed to the down projection
 };
 
-static int num_sms() {
+int num_sms() {
     const int dev = current_device();
     if (g_num_sms[dev] == 0)
         GLMASR_CUDA_CHECK(cudaDeviceGetAttribute(&g_num_sms[dev], cudaDevAttrMultiProcessorCount, dev));

@@ -376,13 +376,7 @@ bool launch_attention64_umma(__nv_bfloat16 *out, int ldo, const __nv_bfloat16 *q
     p.total_items = p.q_tiles * num_q_heads * num_seqs;
     p.causal = causal ? 1 : 0;
     p.scale_log2 = 1.4426950408889634f / 8.0f;
-    static int num_sms = 0;
-    if (num_sms == 0) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        if (cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || num_sms <= 0) num_sms = 148;
-    }
-    const int grid = p.total_items < CTAS_PER_SM * num_sms ? p.total_items : CTAS_PER_SM * num_sms;
+    const int grid = p.total_items < CTAS_PER_SM * num_sms() ? p.total_items : CTAS_PER_SM * num_sms();
     const cudaError_t e = launch_chained(attention64_umma_kernel, dim3(grid), dim3(THREADS64), (size_t)SMEM64, st, p);
     if (e != cudaSuccess) (void)cudaGetLastError();         // refused: the caller goes on to the warp-level kernel
     return e == cudaSuccess;

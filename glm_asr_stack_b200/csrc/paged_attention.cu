@@ -606,12 +606,12 @@ bool launch_paged_decode_split(__nv_bfloat16 *out, int ldo, const __nv_bfloat16 
     // unsplit on a chip that it leaves half empty, the serial walk with RoPE in front of it is the longer way round: a W4A4
     // step of 1 / 9 sequences, 16 query and 4 kv heads, takes 1745 / 1823 us with it and 1710 / 1788 us with two launches,
     // of 19 sequences 1813 and 1817 us, of 40 / 100 sequences 1807 / 1896 and 1857 / 1963 us
-    if (q_packed != nullptr && num_seqs * num_kv_heads <= 74) return false;
-    // three 64 KB CTAs fit an SM: up to 444 in one wave, at least two tiles for every CTA.  A result that is quantised is not
+    if (q_packed != nullptr && num_seqs * num_kv_heads <= num_sms() / 2) return false;
+    // three 64 KB CTAs fit an SM: up to three per SM in one wave, at least two tiles for every CTA.  A result that is quantised is not
     // split: another order of its sums moves values across e2m1 rounding boundaries, and a chain of such layers amplifies it.
     const int tiles = (max_len + kTile - 1) / kTile;
     int splits = 1;
-    while (q_packed == nullptr && splits < 8 && num_seqs * num_kv_heads * splits * 2 <= 444 && tiles >= splits * 4) splits *= 2;
+    while (q_packed == nullptr && splits < 8 && num_seqs * num_kv_heads * splits * 2 <= 3 * num_sms() && tiles >= splits * 4) splits *= 2;
     static PerDevice<bool> configured;
     if (once_per_device(configured, [] { return cudaFuncSetAttribute(paged_decode_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kAttnSmem); }) != cudaSuccess)
         return false;

@@ -557,13 +557,7 @@ bool launch_prefill_attention_umma(__nv_bfloat16 *out, int ldo, const __nv_bfloa
     p.q_sf_chunks = num_q_heads * 2;
     p.q_inv_in = q_packed != nullptr ? 1.0f / q_input_scale : 0.0f;
 
-    static int num_sms = 0;
-    if (num_sms == 0) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        if (cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || num_sms <= 0) num_sms = 148;
-    }
-    const dim3 grid(p.total_items < 2 * num_sms ? p.total_items : 2 * num_sms, 1, 1);
+    const dim3 grid(p.total_items < 2 * num_sms() ? p.total_items : 2 * num_sms(), 1, 1);
 #ifdef GLMASR_EXPERIMENTS
     static int debug = -1;
     if (debug < 0) {

@@ -24,6 +24,7 @@ enum : int { WS_ATTN_DEBUG = 34 };
 void free_all_private_state();
 void tail_forget_scales(const void *w_scales);   // decode_tail.cu: per-CTA re-tiled weight scales (nullptr: all)
 void encoder_forget_all();         // encoder.cu: per-store weight table, re-packed convolution weights, rotary table
+int num_sms();                      // of the current device
 void note_launches(int n);          // launch accounting for kernels started outside api.cu
 size_t tiled_scale_bytes(int rows, int K);   // bytes of the 128x4-tiled scale layout for [rows, K]
 // Cached TMA descriptor of a row-major bf16 matrix [rows, inner] (row pitch in bytes, a multiple of 16; base
