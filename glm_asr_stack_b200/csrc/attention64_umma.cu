@@ -14,8 +14,6 @@
 //   * P goes to its own 64 columns of tensor memory, from where it is the second product's A operand: no shared-memory
 //     stores, no proxy fence.  Scores [0, 128), P [128, 192), output [192, 256): two CTAs per SM;
 //   * V is read as it lies in memory (MN-major B operand).
-// A part of the exponentials runs on the multiply-add pipe instead (kPolyPairs), relative error 2.7e-6 where P is rounded to
-// bf16 (2e-3) right after.
 //   warp 0 TMA producer, warp 1 MMA issuer, warps 2-5 soft-max (thread = query row = TMEM lane).
 #include <cuda_bf16.h>
 #include <math.h>
@@ -77,32 +75,6 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
     const __nv_bfloat162 b = __floats2bfloat162_rn(lo, hi);
     return *reinterpret_cast<const uint32_t *>(&b);
 }
-// 2^x for two values on the multiply-add pipe (x clamped at -126: nothing in a sum whose largest term is near 1).  Split at
-// the nearest integer by the magic number 1.5 * 2^23; minimax polynomial of degree 4 of 2^f on [-1/2, 1/2] (linear
-// programme over 2001 Chebyshev nodes, rounded to float: relative error 2.7e-6 evaluated in float).
-__device__ __forceinline__ void ex2_poly_x2(float &x0, float &x1) {
-    const unsigned long long x = pack_f32x2(fmaxf(x0, -126.0f), fmaxf(x1, -126.0f));
-    const unsigned long long r = add_f32x2(x, pack_f32x2(12582912.0f, 12582912.0f));
-    const unsigned long long i = add_f32x2(r, pack_f32x2(-12582912.0f, -12582912.0f));
-    const unsigned long long f = fma_f32x2(i, pack_f32x2(-1.0f, -1.0f), x);
-    unsigned long long q = fma_f32x2(f, pack_f32x2(0.009567709639668465f, 0.009567709639668465f), pack_f32x2(0.055917490273714066f, 0.055917490273714066f));
-    q = fma_f32x2(q, f, pack_f32x2(0.24024811387062073f, 0.24024811387062073f));
-    q = fma_f32x2(q, f, pack_f32x2(0.6931219696998596f, 0.6931219696998596f));
-    q = fma_f32x2(q, f, pack_f32x2(0.9999992251396179f, 0.9999992251396179f));
-    float r0, r1, q0, q1;
-    unpack_f32x2(r, r0, r1);
-    unpack_f32x2(q, q0, q1);
-    // the integer sits in r's low bits; the magic number's own bits leave at the top of the shift
-    x0 = __int_as_float(__float_as_int(q0) + (__float_as_int(r0) << 23));
-    x1 = __int_as_float(__float_as_int(q1) + (__float_as_int(r1) << 23));
-}
-
-// Pairs of every 16 columns (8 pairs) whose exponentials run on the multiply-add pipe.
-#ifndef KPOLY
-#define KPOLY 0
-#endif
-constexpr int kPolyPairs = KPOLY;
-
 __global__ void __launch_bounds__(THREADS64, CTAS_PER_SM) attention64_umma_kernel(const __grid_constant__ Attn64Params p) {
     extern __shared__ __align__(1024) uint8_t smem[];
     const uint32_t sbase = smem_u32(smem);
@@ -281,12 +253,8 @@ __global__ void __launch_bounds__(THREADS64, CTAS_PER_SM) attention64_umma_kerne
                     for (int c = 0; c < 32; c += 2) {
                         float t0, t1;
                         unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(sr[h][c]), __uint_as_float(sr[h][c + 1])), scale2, neg_m2), t0, t1);
-                        if (((c >> 1) & 7) < kPolyPairs) {
-                            ex2_poly_x2(t0, t1);
-                        } else {
-                            t0 = ex2_sfu(t0);
-                            t1 = ex2_sfu(t1);
-                        }
+                        t0 = ex2_sfu(t0);
+                        t1 = ex2_sfu(t1);
                         sum2 = add_f32x2(sum2, pack_f32x2(t0, t1));
                         pk[c >> 1] = pack_bf16(t0, t1);
                     }
