@@ -27,7 +27,7 @@ extern "C" int count(int device) { return device < 0 ? cleared : set_ups[device]
 def test_once_per_device(tmp_path):
     (tmp_path / "p.cpp").write_text(SOURCE)
     cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
-    subprocess.run(["g++", "-std=c++17", "-shared", "-fPIC", "-I", CSRC, "-I", os.path.join(cuda, "include"), "-o",
+    subprocess.run(["g++", "-std=c++17", "-shared", "-fPIC", "-Wl,-Bsymbolic", "-I", CSRC, "-I", os.path.join(cuda, "include"), "-o",
                     str(tmp_path / "p.so"), str(tmp_path / "p.cpp")], check=True, capture_output=True)
     lib = ctypes.CDLL(str(tmp_path / "p.so"))
     assert lib.use(0, 0) == 0 and lib.use(0, 0) == 0 and lib.count(0) == 1
