@@ -137,6 +137,57 @@ def test_attention_head_dim_64_non_causal(ops, lens):
     assert ops.status() == 0
 
 
+@pytest.mark.parametrize("heads,kv,causal", [(4, 4, False), (4, 4, True), (8, 2, True), (6, 1, False)])
+@pytest.mark.parametrize("lens,q_scale", [([1, 15, 16, 17, 31, 32, 33, 63, 64, 65], 1.0), ([95, 96, 97, 127, 128, 129, 255, 257], 1.0),
+                                          ([700, 0, 131], 6.0)])
+def test_attention_head_dim_64_steps(ops, heads, kv, causal, lens, q_scale):
+    """Sequence ends on both sides of the 16-key steps of the second product, of the 32-column blocks and of the 128-key steps;
+    masked and not, several query heads per key head, scores whose range makes the accumulator be rescaled.  Tolerance: P and
+    the result rounded to bf16."""
+    import decoder_oracle as do
+    from glm_asr_stack_b200 import engine
+    rng = np.random.default_rng(heads + len(lens))
+    hd, offs = 64, np.concatenate([[0], np.cumsum(lens)]).astype(np.int32)
+    T, H, KV = int(offs[-1]), heads * hd, kv * hd
+    qkv = rb(rng, (T, H + 2 * KV))
+    qkv[:, :H] = rb(rng, (T, H), q_scale)
+    buf = to_dev_bf16(qkv)
+    got = bits_of(engine.prefill_attention(buf[:, :H], buf[:, H:H + KV], buf[:, H + KV:], torch.from_numpy(offs).cuda(), max(lens),
+                                           heads, kv, hd, causal))
+    want = do.prefill_attention(qkv[:, :H], qkv[:, H:H + KV], qkv[:, H + KV:], offs[:-1], lens, heads, kv, hd, causal)
+    for off, ln in zip(offs[:-1], lens):
+        if ln:
+            assert o.rel_err(got[off:off + ln], want[off:off + ln]) <= REL_TOL_TIGHT, (off, ln)
+    assert ops.status() == 0
+
+
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("causal", [False, True])
+def test_rows_behind_a_sequence_may_hold_anything(ops, hd, causal):
+    """The tiles of a sequence reach into the rows behind it: NaN and infinities there change no bit of its result."""
+    from glm_asr_stack_b200 import engine
+    gen = torch.Generator(device="cuda").manual_seed(hd)
+    heads, kv, lens = 4, 2, [70, 33, 129, 5, 200, 61]
+    offs = np.concatenate([[0], np.cumsum(lens)]).astype(np.int32)
+    T, H, KV = int(offs[-1]) + 150, heads * hd, kv * hd                # rows of no sequence at the end
+    x = torch.randn((T, H + 2 * KV), generator=gen, device="cuda").to(torch.bfloat16)
+    cu = torch.from_numpy(offs).cuda()
+
+    def run(buf):
+        return engine.prefill_attention(buf[:, :H], buf[:, H:H + KV], buf[:, H + KV:], cu, max(lens), heads, kv, hd, causal)
+
+    want, bad = run(x).clone(), x.clone()
+    for i in (1, 3, 5):
+        bad[offs[i]:offs[i + 1]] = float("nan") if i != 3 else float("inf")
+    bad[offs[-1]:] = float("nan")
+    got = run(bad)
+    for i in (0, 2, 4):
+        assert torch.equal(got[offs[i]:offs[i + 1]].view(torch.int16), want[offs[i]:offs[i + 1]].view(torch.int16)), i
+    bad[offs[5]:offs[6]] = x[offs[5]:offs[6]]                           # the last sequence, poisoned rows behind it only
+    assert torch.equal(run(bad)[offs[5]:offs[6]].view(torch.int16), want[offs[5]:offs[6]].view(torch.int16))
+    assert ops.status() == 0
+
+
 def build_tower(rng, hidden, heads, ffn, layers, mels=128, proj_mid=512, dec_hidden=256):
     """A small random audio tower as a WeightStore plus the oracle's view of it."""
     from glm_asr_stack_b200 import engine
@@ -201,6 +252,27 @@ def test_encoder_forward_packed_small_model(ops, ref):
         r = bits_of(ref.encoder_forward_packed(ws, cfg, to_dev_bf16(h0), lens, offs))
         assert o.rel_err(r[inside], want[inside]) <= REL_TOL_VS_ORACLE        # pins the oracle's layer sequence to the reference
         assert o.rel_err(got[inside], r[inside]) <= REL_TOL_VS_ORACLE
+
+
+def test_encoder_rows_of_no_sequence_have_no_position(ops):
+    """Rows between sequences have no entry in the position list.  Whatever the list's memory held before -- here freed memory
+    full of positions far outside the rotary table -- is not looked up, and the sequences' results do not depend on it."""
+    from glm_asr_stack_b200 import _lib
+    rng = np.random.default_rng(43)
+    ws, cfg, _, _ = build_tower(rng, 256, 4, 512, 1)
+    h0 = to_dev_bf16(rb(rng, (600, 256)))
+    lens, offs = [70, 33, 128], [0, 75, 400]
+    want = ops.encoder_forward_packed(ws, cfg, h0.clone(), lens, offs)
+    torch.cuda.synchronize()
+    _lib.load().glmasr_fp4_cleanup()                                    # the next call allocates its workspaces anew
+    poison = [torch.full((1 << n,), 0x3F000000, dtype=torch.int32, device="cuda") for n in range(18, 25) for _ in range(8)]
+    torch.cuda.synchronize()
+    del poison
+    torch.cuda.empty_cache()
+    got = ops.encoder_forward_packed(ws, cfg, h0.clone(), lens, offs)
+    for off, ln in zip(offs, lens):
+        assert torch.equal(got[off:off + ln].view(torch.int16), want[off:off + ln].view(torch.int16))
+    assert ops.status() == 0
 
 
 def test_encoder_real_width_two_layers(ops, ref):
