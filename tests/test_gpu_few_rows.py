@@ -139,3 +139,59 @@ def test_cluster_route_is_the_faster_one(ops, M, N, K, cluster):
     assert (ops.last_gemm_route()[0] == "cluster") == cluster
     want = x.double() @ w.double().T
     assert float((got - want).norm() / want.norm()) <= REL_TOL_TIGHT
+
+
+@pytest.mark.parametrize("M", [17, 19, 33, 65, 173])
+def test_cluster_epilogues_with_k_split(ops, M):
+    """W4A16 on the cluster GEMM with K really cut (asserted): three ragged segments, gate|up whose gate sums stay in a CTA's own
+    partial tile while its peers read that tile, and a residual added in place.  Each runs twice: the second call finds the bf16
+    copies and fetches them ahead of its dependency wait."""
+    def check_split():
+        assert ops.last_gemm_route()[0] == "cluster" and ops.last_gemm_route()[1] > 1, ops.last_gemm_route()
+
+    for K, ns in ((2048, (2048, 512, 136)), (6144, (264, 40, 512))):
+        x = to_dev_bf16(o.seeded_activation(M, K, M))
+        ws = [rand_fp4(ops, n, K, n + M) for n in ns]
+        wants = [x.double() @ d.to(torch.bfloat16).double().T for _, d in ws]
+        for _ in range(2):
+            out = ops.fp4_linear_fused(ops.MODE_W4A16, x, [w for w, _ in ws]).double()
+            check_split()
+            c = 0
+            for n, want in zip(ns, wants):
+                assert float((out[:, c:c + n] - want).norm() / want.norm()) <= REL_TOL_TIGHT
+                c += n
+        (g, gd), (u, ud) = rand_fp4(ops, 520, K, 1), rand_fp4(ops, 520, K, 2)
+        gw, uw = (0.01 * (x.double() @ d.to(torch.bfloat16).double().T) for d in (gd, ud))
+        g.w_global_scale = u.w_global_scale = 0.0025                    # gates where SiLU bends; the copies round bf16(v) * 0.01 alike
+        want = gw * torch.sigmoid(gw) * uw
+        for _ in range(2):
+            act = ops.fp4_linear_fused(ops.MODE_W4A16, x, [g, u], epilogue=ops.EPI_SILU_GATE).double()
+            check_split()
+            assert float((act - want).norm() / want.norm()) <= REL_TOL_VS_ORACLE
+        (w, _), want = ws[0], wants[0]
+        res = to_dev_bf16(o.seeded_activation(M, ns[0], 9))
+        want = want.to(torch.bfloat16).double() + res.double()
+        for _ in range(2):
+            h = res.clone()
+            ops.fp4_linear_fused(ops.MODE_W4A16, x, [w], epilogue=ops.EPI_RESIDUAL, residual=h, out=h)
+            check_split()
+            assert float((h.double() - want).norm() / want.norm()) <= REL_TOL_TIGHT
+
+
+def test_cluster_share_counts(ops):
+    """K blocks that do not divide by the CTAs that share them (3, 5, 6 and 7 among them, asserted): bf16 weights, bias, GELU."""
+    shares = set()
+    for K, N in ((448, 128), (704, 128), (1984, 640), (3008, 1280), (5120, 1280), (64, 256)):
+        for M in (17, 40, 100):
+            gen = torch.Generator(device="cuda").manual_seed(K + M)
+            x, w = (torch.randn(s, generator=gen, device="cuda").to(torch.bfloat16) for s in ((M, K), (N, K)))
+            b = torch.randn(N, generator=gen, device="cuda").to(torch.bfloat16)
+            want = x.double() @ w.double().T + b.double()
+            got = ops.bf16_linear(x, w, b).double()
+            assert float((got - want).norm() / want.norm()) <= REL_TOL_TIGHT, (M, N, K)
+            name, n = ops.last_gemm_route()
+            shares.add(n if name == "cluster" else 0)
+            got = ops.bf16_linear_gelu(x, w, b).double()
+            want = torch.nn.functional.gelu(want, approximate="tanh")
+            assert float((got - want).norm() / want.norm()) <= REL_TOL_TIGHT, (M, N, K)
+    assert {3, 5, 6, 7, 8} <= shares, shares
