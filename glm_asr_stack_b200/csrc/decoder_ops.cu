@@ -335,9 +335,8 @@ __global__ void rmsnorm_quant_kernel(uint8_t *__restrict__ q_packed, uint8_t *__
 // consecutive 16-element blocks, i.e. 32 contiguous output bytes and one 4-byte group of scales.
 // dim = 2048 * P.
 constexpr int kNormStrip = 32 * 144;      // bytes of shared memory per 2048 elements
-constexpr int kNormWarps = 2;             // rows per CTA: small CTAs end a launch evenly (eight warps: 27.8 us for 10000 rows, two: 26)
-template <int P>
-__global__ void __launch_bounds__(kNormWarps * 32) rmsnorm_quant_warp_kernel(uint8_t *__restrict__ q_packed, uint8_t *__restrict__ q_sf,
+template <int P, int W>                   // W: rows (warps) per CTA
+__global__ void __launch_bounds__(W * 32) rmsnorm_quant_warp_kernel(uint8_t *__restrict__ q_packed, uint8_t *__restrict__ q_sf,
                                                                 int sf_chunks, const __nv_bfloat16 *__restrict__ x,
                                                                 const __nv_bfloat16 *__restrict__ weight, float eps,
                                                                 float inv_in, int rows, __nv_bfloat16 *__restrict__ normed_out) {
@@ -346,7 +345,7 @@ __global__ void __launch_bounds__(kNormWarps * 32) rmsnorm_quant_warp_kernel(uin
     pdl_launch_dependents();
     pdl_wait();
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    const int row = blockIdx.x * kNormWarps + wib;
+    const int row = blockIdx.x * W + wib;
     if (row >= rows) return;
     uint8_t *rs = strips + wib * (P * kNormStrip);
     {
@@ -419,12 +418,23 @@ bool launch_rmsnorm_quant(uint8_t *q_packed, uint8_t *q_sf, const __nv_bfloat16 
         !(input_scale > 0.0f))
         return false;
     if (rows >= 2048 && (dim == 2048 || dim == 4096)) {
-        const dim3 grid((rows + kNormWarps - 1) / kNormWarps);
-        if (dim == 2048) {
-            launch_chained(rmsnorm_quant_warp_kernel<1>, grid, dim3(kNormWarps * 32), (size_t)(kNormWarps * kNormStrip), st, q_packed, q_sf, dim / 64, x,
+        // Eight rows per CTA, four such CTAs per SM.  Two rows per CTA where that would end in a round of a few CTAs: then the
+        // small ones end evenly (5000 rows 14.4 -> 13.9 us, 10000 rows the same alone and 1 - 2 % of a prefill), while elsewhere they
+        // are the slower ones (2048 rows 10.5 / 11.6 us, 4000 rows 11.2 / 13.0, 8000 rows 17.8 / 19.2, 20000 rows 42.5 / 43.8).
+        const int ctas = (rows + 7) / 8, round = 4 * num_sms();
+        if (dim == 2048 && ctas > round && ctas % round != 0 && ctas % round <= round / 8) {
+            launch_chained(rmsnorm_quant_warp_kernel<1, 2>, dim3((rows + 1) / 2), dim3(64), (size_t)(2 * kNormStrip), st, q_packed, q_sf,
+                           dim / 64, x, weight, eps, 1.0f / input_scale, rows, normed_out);
+        } else if (dim == 2048) {
+            launch_chained(rmsnorm_quant_warp_kernel<1, 8>, dim3(ctas), dim3(256), (size_t)(8 * kNormStrip), st, q_packed, q_sf, dim / 64, x,
                            weight, eps, 1.0f / input_scale, rows, normed_out);
         } else {
-            launch_chained(rmsnorm_quant_warp_kernel<2>, grid, dim3(kNormWarps * 32), (size_t)(2 * kNormWarps * kNormStrip), st, q_packed, q_sf, dim / 64, x,
+            static PerDevice<bool> configured;
+            const cudaError_t ready = once_per_device(configured, [] {
+                return cudaFuncSetAttribute(rmsnorm_quant_warp_kernel<2, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, 16 * kNormStrip);
+            });
+            if (ready != cudaSuccess) return false;
+            launch_chained(rmsnorm_quant_warp_kernel<2, 8>, dim3(ctas), dim3(256), (size_t)(16 * kNormStrip), st, q_packed, q_sf, dim / 64, x,
                            weight, eps, 1.0f / input_scale, rows, normed_out);
         }
         return true;

@@ -186,6 +186,12 @@ def test_rmsnorm_quant_equals_norm_then_quantiser(ops, rows, dim):
     assert np.array_equal(got_pk.cpu().numpy(), opk)
 
 
+@pytest.mark.parametrize("rows", [4736, 4737, 5279, 5329, 9999])
+def test_rmsnorm_quant_rows_per_cta(ops, rows):
+    """Both sides of the rule that picks eight or two rows per CTA (148 SMs), odd rows in the last one."""
+    test_rmsnorm_quant_equals_norm_then_quantiser(ops, rows, 2048)
+
+
 def test_embedding_lookup(ops):
     rng = np.random.default_rng(7)
     table = rnd_bits(rng, (100, 256))
