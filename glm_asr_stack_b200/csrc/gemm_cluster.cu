@@ -146,7 +146,8 @@ __global__ void __launch_bounds__(kCgThreads, 2) cluster_gemm_kernel(const __gri
         }
         if (leader) umma_commit(done);
         // this warp polls, the others sleep at the barrier below
-        if (!mbar_wait_warp(done, 0, abort_word, ST_TIMEOUT_EPILOGUE) || !ok) let_copies_land();
+        const bool fin = mbar_wait_warp(done, 0, abort_word, ST_TIMEOUT_EPILOGUE);
+        if (__builtin_expect(!(fin && ok), 0)) let_copies_land();
     }
     pdl_wait();                         // residual, bias and out belong to the preceding kernels until here
     __syncthreads();                    // the ring is dead: every load of it has been consumed by a completed MMA
