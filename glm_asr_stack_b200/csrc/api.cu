@@ -802,9 +802,9 @@ static int run_fused(const FusedArgs &a) {
 #endif
     p.num_m_tiles = (a.M + 127) / 128;
     p.n_out = total_out_cols(a);
-    // W4A4 weights and their re-tiled scales are read-only for every kernel that signals its dependents early:
-    // the only writer, the one-time scale re-tiling, is launched as an ordinary kernel and therefore completes
-    // before anything behind it starts.  So the producer may fetch them ahead of the dependency wait.
+    // The producer may fetch W4A4 weights and their re-tiled scales ahead of the dependency wait: a weight changes only together
+    // with glmasr_fp4_forget (its scales are cached by address), and the first use after that re-tiles them with an ordinary
+    // launch that starts when everything before it -- the weight's writer -- has completed and signals nobody early.
     p.early_weights = (a.mode == GEMM_W4A4 && pdl_enabled()) ? 1 : 0;
 
     // operand A

@@ -2,7 +2,8 @@
 // causal mask) on the tcgen05 tensor cores: per sequence softmax(Q K^T / 8 [+ causal mask]) V, the arithmetic of
 // prefill_attention_umma.cu.
 //
-// With 64 dims a score costs 256 multiply-adds of tensor work and one exponential, so the special-function unit (16 per
+// Sixteen sequences of 1500 rows, 20 heads: 382 -> 302 us (the head_dim 128 kernel run at 64, with its launch that transposed V,
+// before).  With 64 dims a score costs 256 multiply-adds of tensor work and one exponential, so the special-function unit (16 per
 // clock and SM) is the bound: 0.75 G exponentials per layer of 16 full windows are 319 k cycles of it.  The head_dim 128
 // kernel run at 64 (64 keys a step) took 616 k: about 950 cycles of every soft-max step are not exponentials -- tensor-memory
 // load, maximum, hand-overs -- and two warps per scheduler cannot hide them behind each other's 512.  Four CTAs per SM with a

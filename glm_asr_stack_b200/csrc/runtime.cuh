@@ -57,7 +57,7 @@ void profile_bracket_end();
 // A chain of 5-40 us kernels on one stream pays a few microseconds per kernel boundary (launch
 // latency, block scheduling, set-up code).  Kernels launched through launch_chained() may become
 // resident while their predecessor is still draining: each of them calls pdl_launch_dependents()
-// first thing and pdl_wait() before it touches global memory, and pdl_wait() returns only when
+// first thing and pdl_wait() before it touches global memory (weights apart, below), and pdl_wait() returns only when
 // every preceding kernel of the stream has completed and its writes are visible, so data
 // dependencies are exactly those of an ordinary stream.  GLMASR_PDL=0 turns the attribute off.
 bool pdl_enabled();

@@ -38,10 +38,14 @@ void fp4_dequant_to_bf16(uint16_t *out, const uint8_t *packed_w, const uint8_t *
 
 /* Infer-engine/include/cuda_kernels.h:80-89, Infer-engine/cuda/kernels.cu:1297-1318.
  * W4A16: out[M,N] = bf16(x[M,K] * dequant(W)[N,K]^T (+ bias)), fp32 accumulation.
- * The reference materialises the bf16 weight in weight_scratch on every call.  Here, below
- * 1024 rows (decode), the weight is dequantised inside the GEMM and weight_scratch is left
- * untouched; from 1024 rows (prefill) it is dequantised once per call into weight_scratch
- * (a private workspace if NULL), exactly like the reference, and a bf16 GEMM follows.
+ * The reference materialises the bf16 weight in weight_scratch on every call.  Here up to 16
+ * rows run on the packed weight as it is stored, larger calls on a bf16 copy that is made on
+ * first use and kept (GLMASR_W4A16_RESIDENT_MB bounds the copies).  Where no copy is kept, the
+ * weight is dequantised inside the GEMM below 1024 rows, and from 1024 rows on once per call into
+ * weight_scratch (a private workspace if NULL), exactly like the reference, with a bf16 GEMM behind it.
+ * The route, and with it the order in which a row's products are summed in fp32, depends on M; below 17
+ * rows the weights are exact where the copies round lut * scale * global to bf16 (both differ from the
+ * reference by no more than its own rounding).
  * prequant_scratch ([M,K] bf16) is written only when pre_quant_scale != NULL, as in the
  * reference.  handle is ignored (no cuBLAS). */
 void fp4_linear(void *handle, uint16_t *out, uint16_t *weight_scratch, uint16_t *prequant_scratch,
@@ -118,7 +122,9 @@ void paged_decode_attention(uint16_t *out, const uint16_t *query, const uint16_t
  * (nvfp4_linear) while the same-input pairs k|v and gate|up stay W4A16 (the reference's fused pair,
  * Infer-engine/cuda/decoder.cu:923-978, always dequantises), unless a pair carries a pre_quant_scale and is
  * therefore run one projection at a time.  GLMASR_NVFP4_PAIRS=1 (additive, not in the reference) runs the
- * pairs in W4A4 too. */
+ * pairs in W4A4 too.  W4A16 projections and their attention split K and the context by the size of the batch, so
+ * a sequence's result may differ in its last bits with what else is in the batch (all-W4A4 steps do not split).
+ * Rows may share pages and attend to tokens that other rows of the same step write. */
 void decoder_decode_step_batched(void *handle, const void *ws, uint16_t **query_ptrs, void *pool, void *bts,
                                  int *d_seq_lens, int *h_seq_lens, int num_seqs, int *seq_indices,
                                  uint16_t *dequant_buf, const void *cfg);
