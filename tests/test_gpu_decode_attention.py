@@ -133,3 +133,61 @@ def test_rows_that_read_what_other_rows_write(mode):
     r = subprocess.run([sys.executable, "-c", code], env=dict(os.environ, **tgd.MODE_ENV[mode]), capture_output=True,
                        text=True, timeout=600)
     assert r.returncode == 0 and "RESULT" in r.stdout, r.stdout[-4000:] + r.stderr[-4000:]
+
+
+def run_setup(mode):
+    """The set-up of a step in one launch (parameters for 32 or 256 rows) and its copies behind that: rows in one block, rows
+    scattered over memory in any order, rows that are not 16-byte aligned.  Hidden rows, lengths and caches get equal bits."""
+    from glm_asr_stack_b200 import _lib, engine, ops
+    rng = np.random.default_rng(41)
+    ws, cfg, layers, fn, (H, F, QH, KVH, HD, L) = tgd.build_toy_model(rng, 1100, "plain")
+    bs, errs = 16, {}
+    for n in (1, 32, 33, 256, 257):
+        ctx = [(13 * i) % 37 for i in range(n)]
+        cached, num_blocks = np.array(ctx, np.int32), sum(c // bs + 1 for c in ctx)
+        perm = rng.permutation(num_blocks).tolist()
+        tables = [[perm.pop() for _ in range(c // bs + 1)] for c in ctx]
+        bt_np = np.full((n, 4), -1, np.int32)
+        for i, t in enumerate(tables):
+            bt_np[i, :len(t)] = t
+        kc0, vc0 = (tgd.rnd_bits(rng, (L, num_blocks * bs, KVH * HD)) for _ in range(2))
+        hidden = tgd.rnd_bits(rng, (n, H))
+        order = rng.permutation(n).tolist()
+        results = []
+        for layout in ("block", "scattered", "unaligned"):
+            pool = engine.KVPool(num_blocks, bs, L, KVH, HD, max_seqs=n, max_blocks_per_seq=4)
+            bts = engine.BlockTables(pool, tables)
+            pool.k.copy_(to_dev_bf16(kc0).view(pool.k.shape))
+            pool.v.copy_(to_dev_bf16(vc0).view(pool.v.shape))
+            off, pitch = (1, H + 3) if layout == "unaligned" else (0, H if layout == "block" else H + 64)
+            at = order if layout == "scattered" else list(range(n))
+            buf = torch.zeros(n * pitch + 8, dtype=torch.bfloat16, device="cuda")
+            rows = [buf[off + at[i] * pitch:off + at[i] * pitch + H] for i in range(n)]
+            for r, h in zip(rows, to_dev_bf16(hidden)):
+                r.copy_(h)
+            d_lens, h_lens = torch.from_numpy(cached.copy()).cuda(), (ctypes.c_int * n)(*ctx)
+            ptrs = (ctypes.c_void_p * n)(*[r.data_ptr() for r in rows])
+            _lib.load().decoder_decode_step_batched(None, ctypes.byref(ws.c), ptrs, ctypes.byref(pool.c), bts.arr,
+                                                    ctypes.c_void_p(d_lens.data_ptr()), h_lens, n, None, None, ctypes.byref(cfg))
+            torch.cuda.synchronize()
+            assert ops.status() == 0
+            assert list(h_lens) == (cached + 1).tolist() == d_lens.cpu().tolist()
+            results.append((torch.stack(rows), pool.k.clone(), pool.v.clone()))
+        for other in results[1:]:
+            for a, b in zip(results[0], other):
+                assert torch.equal(a.view(torch.int16), b.view(torch.int16)), n
+        slots = np.array([bt_np[i, c // bs] * bs + c % bs for i, c in enumerate(ctx)], np.int64)
+        kc, vc = [kc0[l].copy() for l in range(L)], [vc0[l].copy() for l in range(L)]
+        want = do.decode_step(hidden, layers, fn, kc, vc, bt_np, cached, slots, QH, KVH, HD, bs, tgd.oracle_linears(layers, mode))
+        errs[n] = o.rel_err(bits_of(results[0][0]), want)
+        assert errs[n] <= REL_TOL_VS_ORACLE, errs
+    return errs
+
+
+@pytest.mark.parametrize("mode", ["w4a16", "all_w4a4"])
+def test_step_setup_layouts(mode):
+    code = ("import sys; sys.path[:0]=[%r,%r,%r]; import test_gpu_decode_attention as t; print('RESULT', t.run_setup(%r))"
+            % (ROOT, os.path.join(ROOT, "oracle"), os.path.join(ROOT, "tests"), mode))
+    r = subprocess.run([sys.executable, "-c", code], env=dict(os.environ, **tgd.MODE_ENV[mode]), capture_output=True,
+                       text=True, timeout=600)
+    assert r.returncode == 0 and "RESULT" in r.stdout, r.stdout[-4000:] + r.stderr[-4000:]
